@@ -313,7 +313,7 @@ LbmView<T> lbm_view(hc_handle* h, int src, int fcur) {
   L.unode = (T*)h->unode;
   L.stamp = h->stamp;
   L.reverse = src;  // alternates with the buffer parity
-  L.omega = (T)(1.0 / h->u.tau);
+  L.ck = hcd::collide_constants<T>((T)(1.0 / h->u.tau));
   for (int c = 0; c < hcd::MAX_WALL_CLASSES; ++c)
     for (int a = 0; a < 3; ++a) L.uw[c][a] = (T)h->uw[c][a];
   L.status = h->status;

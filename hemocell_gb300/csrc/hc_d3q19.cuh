@@ -198,13 +198,6 @@ __device__ __forceinline__ void pull_inline(const LbmView<T>& L, const T* __rest
   const int cxm = X == 0 ? nx : 0, cxp = X == nx - 1 ? -nx : 0;
   const int cym = Y == 0 ? nxy : 0, cyp = Y == L.ny - 1 ? -nxy : 0;
   const int czm = Z == 0 ? N : 0, czp = Z == L.nz - 1 ? -N : 0;
-  const uint32_t cls = (m >> NB_CLASS_SHIFT) & (MAX_WALL_CLASSES - 1);
-  T ux = T(0), uy = T(0), uz = T(0);
-  if constexpr (MW) {
-    ux = L.uw[cls][0];
-    uy = L.uw[cls][1];
-    uz = L.uw[cls][2];
-  }
   f[0] = HC_IN(L.status, n, N) ? __ldg(src + n) : T(0);
 #pragma unroll
   for (int j = 1; j < 19; ++j) {
@@ -213,12 +206,20 @@ __device__ __forceinline__ void pull_inline(const LbmView<T>& L, const T* __rest
     const int corr = (cxi(j) > 0 ? cxm : (cxi(j) < 0 ? cxp : 0)) + (cyi(j) > 0 ? cym : (cyi(j) < 0 ? cyp : 0)) +
                      (czi(j) > 0 ? czm : (czi(j) < 0 ? czp : 0));
     const int k = bb ? i * N + n : n + L.off[j] + corr;
-    const T v = HC_IN(L.status, k, 19LL * N) ? __ldg(src + k) : T(0);
-    if constexpr (MW) {
-      const T cuw = T(cxi(i)) * ux + T(cyi(i)) * uy + T(czi(i)) * uz;
-      f[j] = bb ? v - T(6.0 * wi(i)) * cuw : v;
-    } else {
-      f[j] = v;
+    f[j] = HC_IN(L.status, k, 19LL * N) ? __ldg(src + k) : T(0);
+  }
+  if constexpr (MW) {
+    // the moving-wall term, only in warps that hold a bounce-back link: at
+    // every node it would cost a third of the node's FP64 instructions
+    if (m & NB_LINKS) {
+      const uint32_t cls = (m >> NB_CLASS_SHIFT) & (MAX_WALL_CLASSES - 1);
+      const T ux = L.uw[cls][0], uy = L.uw[cls][1], uz = L.uw[cls][2];
+#pragma unroll
+      for (int j = 1; j < 19; ++j) {
+        const int i = oppi(j);
+        const T t = f[j] - T(6.0 * wi(i)) * cdot(cxi(i), cyi(i), czi(i), ux, uy, uz);
+        f[j] = (m >> (i - 1)) & 1u ? t : f[j];
+      }
     }
   }
 }

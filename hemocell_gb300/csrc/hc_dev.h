@@ -16,10 +16,27 @@ namespace hcd {
 
 constexpr uint32_t NB_SOLID = 1u << 23;     // node itself is a wall node
 constexpr uint32_t NB_INTERIOR = 1u << 22;  // fluid, no bounce-back link, on no periodic face
+constexpr uint32_t NB_LINKS = (1u << 18) - 1;  // bit i - 1: direction i bounces back
 constexpr int NB_CLASS_SHIFT = 24;        // wall class of the bounce-back neighbours
 constexpr uint32_t NB_CLASS_MIXED = 255;  // neighbours of differing wall class
 constexpr int MAX_WALL_CLASSES = 16;
 constexpr int MAX_TYPES = 8;
+
+// Constants of the Guo-forced BGK collision that depend on omega alone: formed
+// once on the host, as every FP64 instruction that a thread spends on them
+// costs the FP64 pipe 16 cycles a warp.
+template <typename T>
+struct CollideK {
+  T om, om1, hs;  // omega, 1 - omega, 1 - omega/2
+  T gF;      // -3 (1 - omega/2)
+  T am, aF;  // omega 4.5/18 and (1 - omega/2) 9/18
+  T bm, bF;  // omega 3/18 and (1 - omega/2) 3/18
+};
+template <typename T>
+inline CollideK<T> collide_constants(T om) {
+  const T hs = T(1) - T(0.5) * om;
+  return {om, T(1) - om, hs, T(-3) * hs, T(0.25) * om, T(0.5) * hs, om / T(6), hs / T(6)};
+}
 
 template <typename T>
 struct LbmView {
@@ -39,7 +56,7 @@ struct LbmView {
   T* unode;                      // [3][N] velocity of tagged nodes
   uint32_t* stamp;               // device step stamp (advanced by interp_advance)
   int reverse;                   // sweep the lattice from the last z-plane down
-  T omega;
+  CollideK<T> ck;
   T uw[MAX_WALL_CLASSES][3];
   // 32-bit pull offsets, valid when 19 N < 2^31 (fast != 0): population j of
   // an interior node n (no wrap, no bounce-back link) is fsrc[n + off[j]]

@@ -25,40 +25,79 @@ __device__ __forceinline__ void collide_store(const LbmView<T>& L, Idx n, int Z,
   if constexpr (KEEP) pol = l2_policy_evict_last();
   T rhoBar, jx, jy, jz;
   moments(f, rhoBar, jx, jy, jz);
-  const T rho = T(1) + rhoBar;
-  const T invRho = T(1) / rho;
-  const T ux = (jx + T(0.5) * Fx) * invRho;
-  const T uy = (jy + T(0.5) * Fy) * invRho;
-  const T uz = (jz + T(0.5) * Fz) * invRho;
-  const T uu = ux * ux + uy * uy + uz * uz;
-  const T uF = ux * Fx + uy * Fy + uz * Fz;
-  const T om = L.omega;
-  const T om1 = T(1) - om;
-  const T hs = T(1) - T(0.5) * om;
-  const T A = rhoBar - T(1.5) * rho * uu;  // even equilibrium part without w
-  const T B = T(4.5) * rho;
-  const T K = T(3) * rho * om;
-  const T G = T(-3) * hs * uF;
-  const T H = T(9) * hs;
-  const T Lc = T(3) * hs;
-  const T w1 = T(1.0 / 18.0);
-  const T Aw1 = om * w1 * A, Bw1 = om * w1 * B, Gw1 = w1 * G, Hw1 = w1 * H, Kw1 = w1 * K, Lw1 = w1 * Lc;
-  const T Aw2 = T(0.5) * Aw1, Bw2 = T(0.5) * Bw1, Gw2 = T(0.5) * Gw1, Hw2 = T(0.5) * Hw1, Kw2 = T(0.5) * Kw1,
-          Lw2 = T(0.5) * Lw1;
+  if constexpr (sizeof(T) == 8) {
+    // FP64: the FP64 pipe bounds this kernel, so the fewest operations.  With
+    // m = rho u = j + F/2 and opposite velocities c, -c of weight w, the
+    // equilibrium and Guo source of the pair are P + Q and P - Q:
+    //   P = w [om (rhoBar - 1.5 m.u) - 3 hs u.F] + (c.u) (c.a)
+    //   Q = c.b,   a = w (4.5 om m + 9 hs F),   b = w (3 om m + 3 hs F)
+    // (hs = 1 - om/2).  Both quadratic terms of P share the factor c.u, so a
+    // diagonal pair costs three sums and one multiply-add for P and Q instead
+    // of two sums, two products and three multiply-adds: 146 FP64 instructions
+    // a node where the expression by equilibrium and source took 206.  The
+    // 64x64x256 pipe's (x, y)-block kernel goes from 371 to 273 us, the 150^3
+    // Couette box's (moving walls) from 1620 to 967 us.  FP32 keeps the longer
+    // form below: its rounding is the smaller one of the two (velocity error of
+    // 600 steps 4.7e-6 against 7.5e-6), and arithmetic does not bound it.
+    const T invRho = T(1) / (T(1) + rhoBar);
+    const T mx = jx + T(0.5) * Fx, my = jy + T(0.5) * Fy, mz = jz + T(0.5) * Fz;
+    const T ux = mx * invRho, uy = my * invRho, uz = mz * invRho;
+    const T mu = mx * ux + my * uy + mz * uz;
+    const T uF = ux * Fx + uy * Fy + uz * Fz;
+    const CollideK<T>& k = L.ck;
+    const T even = k.om * (rhoBar - T(1.5) * mu) + k.gF * uF;
+    const T P1 = T(1.0 / 18.0) * even, P2 = T(0.5) * P1;
+    const T a1x = k.am * mx + k.aF * Fx, a1y = k.am * my + k.aF * Fy, a1z = k.am * mz + k.aF * Fz;
+    const T b1x = k.bm * mx + k.bF * Fx, b1y = k.bm * my + k.bF * Fy, b1z = k.bm * mz + k.bF * Fz;
+    const T a2x = T(0.5) * a1x, a2y = T(0.5) * a1y, a2z = T(0.5) * a1z;
+    const T b2x = T(0.5) * b1x, b2y = T(0.5) * b1y, b2z = T(0.5) * b1z;
 
-  st_pop<KEEP>(L.fdst + n, om1 * f[0] + T(1.0 / 3.0) * (om * A + G), pol);
+    st_pop<KEEP>(L.fdst + n, k.om1 * f[0] + T(1.0 / 3.0) * even, pol);
 #pragma unroll
-  for (int i = 1; i <= 9; ++i) {
-    const int j = i + 9;  // c = c_j
-    const T cu = cdot(cxi(j), cyi(j), czi(j), ux, uy, uz);
-    const T cF = cdot(cxi(j), cyi(j), czi(j), Fx, Fy, Fz);
-    const bool axis = (wi(j) > 1.0 / 20.0);
-    const T Aw = axis ? Aw1 : Aw2, Bw = axis ? Bw1 : Bw2, Gw = axis ? Gw1 : Gw2;
-    const T Hw = axis ? Hw1 : Hw2, Kw = axis ? Kw1 : Kw2, Lw = axis ? Lw1 : Lw2;
-    const T P = (Bw * (cu * cu) + Aw) + (Hw * (cu * cF) + Gw);
-    const T Q = Kw * cu + Lw * cF;
-    st_pop<KEEP>(L.fdst + j * N + n, om1 * f[j] + (P + Q), pol);
-    st_pop<KEEP>(L.fdst + i * N + n, om1 * f[i] + (P - Q), pol);
+    for (int i = 1; i <= 9; ++i) {
+      const int j = i + 9;  // c = c_j
+      const bool axis = (wi(j) > 1.0 / 20.0);
+      const T cu = cdot(cxi(j), cyi(j), czi(j), ux, uy, uz);
+      const T ca = axis ? cdot(cxi(j), cyi(j), czi(j), a1x, a1y, a1z) : cdot(cxi(j), cyi(j), czi(j), a2x, a2y, a2z);
+      const T Q = axis ? cdot(cxi(j), cyi(j), czi(j), b1x, b1y, b1z) : cdot(cxi(j), cyi(j), czi(j), b2x, b2y, b2z);
+      const T P = cu * ca + (axis ? P1 : P2);
+      st_pop<KEEP>(L.fdst + j * N + n, k.om1 * f[j] + (P + Q), pol);
+      st_pop<KEEP>(L.fdst + i * N + n, k.om1 * f[i] + (P - Q), pol);
+    }
+  } else {
+    const T rho = T(1) + rhoBar;
+    const T invRho = T(1) / rho;
+    const T ux = (jx + T(0.5) * Fx) * invRho;
+    const T uy = (jy + T(0.5) * Fy) * invRho;
+    const T uz = (jz + T(0.5) * Fz) * invRho;
+    const T uu = ux * ux + uy * uy + uz * uz;
+    const T uF = ux * Fx + uy * Fy + uz * Fz;
+    const T om = L.ck.om, om1 = L.ck.om1, hs = L.ck.hs;
+    const T A = rhoBar - T(1.5) * rho * uu;  // even equilibrium part without w
+    const T B = T(4.5) * rho;
+    const T K = T(3) * rho * om;
+    const T G = T(-3) * hs * uF;
+    const T H = T(9) * hs;
+    const T Lc = T(3) * hs;
+    const T w1 = T(1.0 / 18.0);
+    const T Aw1 = om * w1 * A, Bw1 = om * w1 * B, Gw1 = w1 * G, Hw1 = w1 * H, Kw1 = w1 * K, Lw1 = w1 * Lc;
+    const T Aw2 = T(0.5) * Aw1, Bw2 = T(0.5) * Bw1, Gw2 = T(0.5) * Gw1, Hw2 = T(0.5) * Hw1, Kw2 = T(0.5) * Kw1,
+            Lw2 = T(0.5) * Lw1;
+
+    st_pop<KEEP>(L.fdst + n, om1 * f[0] + T(1.0 / 3.0) * (om * A + G), pol);
+#pragma unroll
+    for (int i = 1; i <= 9; ++i) {
+      const int j = i + 9;  // c = c_j
+      const T cu = cdot(cxi(j), cyi(j), czi(j), ux, uy, uz);
+      const T cF = cdot(cxi(j), cyi(j), czi(j), Fx, Fy, Fz);
+      const bool axis = (wi(j) > 1.0 / 20.0);
+      const T Aw = axis ? Aw1 : Aw2, Bw = axis ? Bw1 : Bw2, Gw = axis ? Gw1 : Gw2;
+      const T Hw = axis ? Hw1 : Hw2, Kw = axis ? Kw1 : Kw2, Lw = axis ? Lw1 : Lw2;
+      const T P = (Bw * (cu * cu) + Aw) + (Hw * (cu * cF) + Gw);
+      const T Q = Kw * cu + Lw * cF;
+      st_pop<KEEP>(L.fdst + j * N + n, om1 * f[j] + (P + Q), pol);
+      st_pop<KEEP>(L.fdst + i * N + n, om1 * f[i] + (P - Q), pol);
+    }
   }
   FieldLayout<T>::store(L.Fnext, N, n, L.bodyz[Z], L.bodyz[L.nz + Z], L.bodyz[2 * L.nz + Z]);
 }
@@ -73,11 +112,16 @@ __device__ __forceinline__ void collide_store(const LbmView<T>& L, Idx n, int Z,
 // (pull_rows); otherwise each thread pulls directly from global memory.
 // The sweep direction alternates every step (L.reverse): a pass then starts
 // on the planes the previous pass wrote last, which are still in L2.
+// Five blocks of 256 threads an SM in FP32 (48 registers; the moving-wall
+// variants take 60 and four blocks otherwise), three in FP64 (80).
+template <typename T>
+constexpr int kCollideBlocks = sizeof(T) == 4 ? 5 : 3;
+
 // V (direct pull with I32 only): bit 0 interior nodes take pull_interior,
 // bit 1 evict-last population stores, bit 2 moving walls (clear: every wall
 // class is at rest and pull_inline drops the moving-wall term).
 template <typename T, bool ROWS, bool I32, int V = 4>
-__global__ void __launch_bounds__(256) k_collide_stream(const LbmView<T> L) {
+__global__ void __launch_bounds__(256, kCollideBlocks<T>) k_collide_stream(const LbmView<T> L) {
   pdl_wait();
   if (L.bump_stamp && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0)
     *L.stamp += 1;
@@ -131,7 +175,7 @@ __device__ __forceinline__ void unpack_node(uint32_t c, int& X, int& Y, int& Z) 
 // V as for k_collide_stream (bit 0 interior pull, bit 1 evict-last stores,
 // bit 2 moving walls).
 template <typename T, int V>
-__global__ void __launch_bounds__(256) k_collide_stream_fluid(const LbmView<T> L) {
+__global__ void __launch_bounds__(256, kCollideBlocks<T>) k_collide_stream_fluid(const LbmView<T> L) {
   pdl_wait();
   if (L.bump_stamp && blockIdx.x == 0 && threadIdx.x == 0) *L.stamp += 1;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -401,6 +445,22 @@ cudaError_t launch_collide_stream(const LbmView<T>& L, int bx, int by, cudaStrea
 // tagged by this step's stencils (Palabos computeVelocity for Guo forcing,
 // core/hemoCellParticleField.cpp:833); L.fsrc is the post-collision state,
 // L.Fcur the force of that collision.
+// FP64 takes one reciprocal of rho for the three components, as the collision
+// does: an FP64 division is about ten instructions of the pipe that bounds the
+// kernel.
+template <typename T>
+__device__ __forceinline__ void store_velocity(const LbmView<T>& L, long long n, T rhoBar, T jx, T jy, T jz, T Fx, T Fy,
+                                               T Fz) {
+  const T rho = T(1) + rhoBar;
+  const T mx = jx + T(0.5) * Fx, my = jy + T(0.5) * Fy, mz = jz + T(0.5) * Fz;
+  if constexpr (sizeof(T) == 8) {
+    const T inv = T(1) / rho;
+    FieldLayout<T>::store(L.unode, L.N, n, mx * inv, my * inv, mz * inv);
+  } else {
+    FieldLayout<T>::store(L.unode, L.N, n, mx / rho, my / rho, mz / rho);
+  }
+}
+
 template <typename T, bool I32>
 __global__ void __launch_bounds__(256) k_node_velocity(const LbmView<T> L) {
   pdl_wait();
@@ -418,9 +478,7 @@ __global__ void __launch_bounds__(256) k_node_velocity(const LbmView<T> L) {
   T rhoBar, jx, jy, jz, Fx, Fy, Fz;
   moments(f, rhoBar, jx, jy, jz);
   FieldLayout<T>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
-  const T rho = T(1) + rhoBar;
-  FieldLayout<T>::store(L.unode, L.N, n, (jx + T(0.5) * Fx) / rho, (jy + T(0.5) * Fy) / rho,
-                        (jz + T(0.5) * Fz) / rho);
+  store_velocity(L, n, rhoBar, jx, jy, jz, Fx, Fy, Fz);
   pdl_trigger();
 }
 template <typename T>
@@ -439,9 +497,7 @@ __global__ void __launch_bounds__(256) k_node_velocity_fluid(const LbmView<T> L)
   T rhoBar, jx, jy, jz, Fx, Fy, Fz;
   moments(f, rhoBar, jx, jy, jz);
   FieldLayout<T>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
-  const T rho = T(1) + rhoBar;
-  FieldLayout<T>::store(L.unode, L.N, n, (jx + T(0.5) * Fx) / rho, (jy + T(0.5) * Fy) / rho,
-                        (jz + T(0.5) * Fz) / rho);
+  store_velocity(L, n, rhoBar, jx, jy, jz, Fx, Fy, Fz);
   pdl_trigger();
 }
 
@@ -461,9 +517,7 @@ __device__ __forceinline__ void node_velocity_at(const LbmView<T>& L, int n) {
   T rhoBar, jx, jy, jz, Fx, Fy, Fz;
   moments(f, rhoBar, jx, jy, jz);
   FieldLayout<T>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
-  const T rho = T(1) + rhoBar;
-  FieldLayout<T>::store(L.unode, L.N, n, (jx + T(0.5) * Fx) / rho, (jy + T(0.5) * Fy) / rho,
-                        (jz + T(0.5) * Fz) / rho);
+  store_velocity(L, n, rhoBar, jx, jy, jz, Fx, Fy, Fz);
 }
 
 template <typename T>
@@ -529,9 +583,7 @@ __global__ void __launch_bounds__(256) k_node_velocity_dense(const LbmView<T> L)
   T rhoBar, jx, jy, jz, Fx, Fy, Fz;
   moments(f, rhoBar, jx, jy, jz);
   FieldLayout<T>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
-  const T rho = T(1) + rhoBar;
-  FieldLayout<T>::store(L.unode, L.N, n, (jx + T(0.5) * Fx) / rho, (jy + T(0.5) * Fy) / rho,
-                        (jz + T(0.5) * Fz) / rho);
+  store_velocity(L, n, rhoBar, jx, jy, jz, Fx, Fy, Fz);
   pdl_trigger();
 }
 
