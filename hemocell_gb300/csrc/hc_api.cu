@@ -39,6 +39,7 @@ struct TypeSlot {
   std::vector<int> cells;
   int* dcells = nullptr;
   int dcells_cap = 0;
+  bool cluster16 = false;  // the device can hold this type's staged assembly on 16 CTAs a cell
 };
 }  // namespace
 
@@ -99,6 +100,9 @@ struct hc_handle {
   // k1 bx (0: row-staged, blocks of whole x-rows), k1 by, spread bs, ibm bs, mech bs, mech grid,
   // mech variant (0 vertex gather, 1 face/edge scatter)
   int tune[8] = {64, 2, 128, 128, 384, 0, 0, 0};
+  bool tuned = false;  // tune is the caller's (hc_set_tuning, hc_autotune), not the rules' (apply_rules)
+  int sms = 1;         // SMs of the device
+  int staged_limit = 0;  // dynamic shared memory the staged force assembly may take
   // repulsion (setRepulsion / enableBoundaryParticles): constants, cutoffs in
   // lattice units, timescales (0 = off) and device state
   double rep_k = 0, rep_rc = 0, brep_k = 0, brep_rc = 0;
@@ -284,6 +288,12 @@ bool tags_needed(const hc_handle* h, const int* tune) {
   return !((tune[7] & 0x300) == 0x300 && 19LL * h->N < (1LL << 31));
 }
 
+int used_types(const hc_handle* h) {
+  int used = 0;
+  for (const TypeSlot& ts : h->types) used += !ts.cells.empty();
+  return used;
+}
+
 int undo_fused_spread(hc_handle* h);
 
 // A new tuning whose node velocity reads tags, while the spread already fused
@@ -349,6 +359,45 @@ VertexView<T> vertex_view(hc_handle* h) {
   vv.frep_cell = h->rep_every > 0 ? (const T*)h->frep_cell : nullptr;
   vv.frep_wall = h->brep_every > 0 ? (const T*)h->frep_wall : nullptr;
   return vv;
+}
+
+// The launch shapes of a handle whose caller chose none (hc_set_tuning,
+// hc_autotune), from its lattice and cells.  Steps in microseconds, this choice
+// against the other side of the line:
+//   Collide-stream in FP64: over the fluid-node list, as a warp with one fluid
+//   node costs the FP64 pipe as much as a full one (pipe 64x64x256 206 against
+//   273 for the kernel, 150^3 Couette box 904 against 967).
+//   In FP32: (x, y)-blocks, or the list where rows rounded up to warps idle a
+//   twentieth of their lanes (rows of 64: 92 against 96; of 97: 29 against 32; of
+//   181: 65 against 67); evict-last population stores (pipe 92 against 96,
+//   suspension 128^3 241 against 244, elsewhere within 1%).
+//   Node velocity in FP32: every fluid node from one vertex for 24 nodes on (96^3
+//   with 80 RBCs 78 against 81; with 20 65 against 72 the other way), else the
+//   tagged nodes packed into warps from half a million nodes on (128^3 with 6
+//   RBCs 96 against 101; 64^3 with 8 36.9 against 35.8).  In FP64 tagged fluid
+//   nodes (pipe 453; every node 482, packed 449; 50^3 box 94, 109, 96).
+//   Programmatic launch always (32^3 box 28.7 against 30.5; FP64 50^3 box 82
+//   against 94).
+//   Force assembly: variant 2 (see mech_plan).
+void apply_rules(hc_handle* h) {
+  if (h->tuned) return;
+  const int rule[8] = {64, 4, 128, 128, 384, 0, 2, 0x400};
+  std::memcpy(h->tune, rule, sizeof(rule));
+  const bool fast32 = 19LL * h->N < (1LL << 31);
+  const int pad = (h->nx + 31) / 32 * 32 - h->nx;
+  if (h->nfluid > 0 && (h->f64 || 20 * pad >= h->nx)) {
+    h->tune[0] = 128;
+    h->tune[1] = 1;
+    h->tune[7] |= 1;
+  }
+  if (h->f64) {
+    if (h->nfluid > 0) h->tune[7] |= 0x100;
+    return;
+  }
+  if (!fast32) return;
+  h->tune[7] |= 0x2000;
+  if (24LL * h->nvert >= h->N) h->tune[7] |= 0x300;
+  else if (h->N >= 500000) h->tune[7] |= 0x200;
 }
 
 // ----- nbmask: per node, which directions bounce back and the wall class
@@ -428,6 +477,7 @@ int upload_flags(hc_handle* h) {
   }
   h->nfluid = (int)fl.size();
   HC_CUDA(h, cudaStreamSynchronize(h->stream));
+  apply_rules(h);
   return HC_OK;
 }
 
@@ -729,22 +779,127 @@ bool fusable(hc_handle* h) {
   return true;
 }
 
-// Shared memory the force assembly of one cell type takes in a variant: the
-// staged variant when its face and edge terms fit the staged maximum, else
-// the vertex-centric path it falls back to.  FP32: 110 KB, so that two CTAs
-// share an SM; FP64: 200 KB, since the FP64 kernel's registers (144 a thread
-// at 384 threads) already hold one CTA per SM, and an FP64 RBC's terms take
-// 150 KB.
-size_t staged_max(const hc_handle* h) { return (h->f64 ? 200 : 110) * (size_t)1024; }
-size_t mech_smem(const hc_handle* h, const TypeSlot& ts, int variant) {
-  const size_t gather = h->f64 ? hcd::mechanics_smem_bytes<double>(ts.tc.nv) : hcd::mechanics_smem_bytes<float>(ts.tc.nv);
-  if (variant != 2) return gather;
-  const size_t staged = hcd::mechanics_staged_bytes(ts.tc.model, ts.tc.nv, ts.tc.nf, ts.tc.ne, h->f64);
-  return staged <= staged_max(h) ? staged : gather;
+size_t gather_bytes(const hc_handle* h, const TypeSlot& ts, int cluster = 1) {
+  return h->f64 ? hcd::mechanics_smem_bytes<double>(ts.tc.nv, cluster)
+                : hcd::mechanics_smem_bytes<float>(ts.tc.nv, cluster);
+}
+
+// How the force assembly launches the cells of one type (variants 0 and 2).
+// CTAs a cell, a power of two.  FP32: as many as leave every CTA an SM of its
+// own, at most 8.  FP64, whose one pipe an SM bounds it, splits finer, so that
+// the SMs' shares come out even and one CTA's loads fill another's gaps: 2 at
+// least, 4 up to three CTAs an SM (two where other types' CTAs need room beside
+// them: 110 RBCs with 11 platelets and a WBC take 162 us a step on 4 CTAs a
+// cell, some of which then wait for a second wave), 8 up to two.  Either form takes 16 where 8
+// would leave a CTA more than 96 vertices.  Measured in microseconds a step,
+// staged, with the advance and spread in it, n RBCs of 642 vertices on
+// 1 / 2 / 4 / 8 CTAs a cell:
+//   FP64  n = 30: 112 / 61 / 51 / 49    110: 112 / 98 / 90 / 133
+//         n = 220: 199 / 147 / 165 / 220    280: 198 / 187 / 231 / 256
+//   FP32  n = 30: 34 / 30 / 29 / 31     60: 34 / 30 / 36 / 41
+//         n = 110: 35 / 40 / 48 / 54    280: 48 / 79 / 112 / 141
+// Threads, staged: one per face of the CTA's share, 128 to 384 (256 from four
+// CTAs a cell on); the 384 of a whole RBC are two CTAs an SM.
+// An FP32 type whose terms, face by face and edge by edge, took more than 110 KB
+// in one CTA (a 2562-vertex WBC) is assembled vertex by vertex, as is one whose
+// terms do not fit at all and, unless the caller chose the variant, a handful of
+// small cells: they take the same time either way, and the vertex-centric
+// kernel's spread adds in the same order from run to run.
+bool few_small(const hc_handle* h) {
+  if (h->ncells > 16) return false;
+  for (const TypeSlot& ts : h->types)
+    if (!ts.cells.empty() && ts.tc.nv > 256) return false;
+  return true;
+}
+struct MechPlan {
+  bool staged;
+  int cluster, bs;
+  size_t smem;
+};
+MechPlan mech_plan(const hc_handle* h, const TypeSlot& ts) {
+  const long long n = (long long)ts.cells.size();
+  const int nv = ts.tc.nv, nf = ts.tc.nf, ne = ts.tc.ne, model = ts.tc.model;
+  auto bytes = [&](int cs) { return hcd::mechanics_staged_bytes(model, nv, nf, ne, cs, h->f64); };
+  if (h->tune[6] == 1) return {false, 1, h->tune[4], gather_bytes(h, ts)};
+  int cs = 1;
+  if (h->f64) cs = 8 * n <= 2 * h->sms ? 8 : (4 * n <= (used_types(h) > 1 ? 2 : 3) * h->sms ? 4 : 2);
+  else
+    while (cs < 8 && 2 * n * cs <= h->sms) cs *= 2;
+  // with the spread in it, CTAs of one cell add to the same nodes in whatever
+  // order they arrive: a cell that one round of a CTA's threads holds stays whole
+  if (h->p.launch == HC_LAUNCH_BATCHED && nv <= 256) cs = 1;
+  if (cs == 8 && nv > 8 * 96 && 16 * n <= h->sms && ts.cluster16) cs = 16;
+  const size_t whole = 4 * (6 * (size_t)nv + 7 * (size_t)nf + 3 * (size_t)ne * (model == HC_MODEL_PLT_SIMPLE ? 2 : 1)) +
+                       (size_t)nv + 272;
+  if (h->tune[6] == 2 && (h->f64 || (whole <= 110 * 1024 && (h->tuned || !few_small(h))))) {
+    int c = cs;
+    while (c < 8 && bytes(c) > (size_t)h->staged_limit) c *= 2;
+    if (bytes(c) <= (size_t)h->staged_limit) {
+      int bs = std::max(128, std::min(c < 4 ? 384 : 256, ((nf + c - 1) / c + 31) / 32 * 32));
+      if (h->tuned && c == 1) bs = std::min(h->tune[4], 384);
+      return {true, c, bs, bytes(c)};
+    }
+  }
+  const int bs = cs == 1 ? h->tune[4] : std::max(128, std::min(h->tune[4], ((nf + cs - 1) / cs + 31) / 32 * 32));
+  return {false, cs, bs, gather_bytes(h, ts, cs)};
 }
 
 inline void prof_mark(hc_handle* h, int slot) {
   if (h->prof_step >= 0) cudaEventRecord(h->prof_ev[h->prof_step * 6 + slot], h->stream);
+}
+
+// The force assembly of the due types.  Variant 2 with every type due (all_due)
+// runs the types side by side, the one with the most vertices last: a
+// suspension's few large cells would otherwise hold the step up before or behind
+// the red ones (one 2562-vertex WBC took 1550 of the 1557 us of an FP64
+// suspension's force assembly) or, in one launch, make every CTA take their
+// shared memory.  Each launch lets the next start once its CTAs run (programmatic
+// launch), and ends after the one before it; on forked streams the same launches
+// took 300 us a step instead of 250 inside a graph, which puts the large clusters
+// last.  A handful of small cells (few_small) takes one launch.  Otherwise one
+// launch per type, one after another.
+template <typename T>
+int enq_types(hc_handle* h, hcd::MechView<T> M, bool forced, bool all_due) {
+  struct Launch {
+    MechPlan plan;
+    const int* cells;
+    long long n, vertices;
+  };
+  std::vector<Launch> launches;
+  const bool together = h->tune[6] == 2 && all_due;
+  for (const TypeSlot& ts : h->types)
+    if (!ts.cells.empty() && (forced || h->iter % ts.every == 0))
+      launches.push_back({mech_plan(h, ts), ts.dcells, (long long)ts.cells.size(), (long long)ts.cells.size() * ts.tc.nv});
+  if (launches.empty()) return HC_OK;
+  if (together && h->p.launch == HC_LAUNCH_BATCHED && few_small(h)) {
+    Launch one = launches[0];
+    for (const Launch& l : launches) {
+      one.plan.smem = std::max(one.plan.smem, l.plan.smem);
+      one.plan.bs = std::max(one.plan.bs, l.plan.bs);
+    }
+    launches = {{one.plan, h->dcells_all, h->ncells, 0}};
+  } else if (together) {
+    std::stable_sort(launches.begin(), launches.end(),
+                     [](const Launch& a, const Launch& b) { return a.vertices < b.vertices; });
+  }
+  const bool overlap = together && launches.size() > 1;
+  const int pdl = M.L.pdl;
+  for (size_t k = 0; k < launches.size(); ++k) {
+    const Launch& l = launches[k];
+    M.cells = l.cells;
+    M.ncells = (int)l.n;
+    M.dyn_smem = (int)l.plan.smem;
+    M.after_prev = overlap && k > 0;
+    M.before_next = overlap && k + 1 < launches.size();
+    M.L.pdl = pdl || M.after_prev;
+    // an SM configured for small CTAs takes no large one until they end: side by
+    // side all launches run on the same split of the SM's memory (an FP64
+    // suspension's step 222 us against 247 without, 232 at 100 percent)
+    M.carveout = overlap ? 55 : 0;
+    if (l.plan.staged) HC_CUDA(h, hcd::launch_mechanics_staged<T>(M, l.plan.cluster, l.plan.bs, h->stream));
+    else HC_CUDA(h, hcd::launch_mechanics<T>(M, l.plan.cluster, l.plan.bs, 0, h->tune[6] == 1 ? 1 : 0, h->stream));
+  }
+  return HC_OK;
 }
 
 template <typename T>
@@ -759,31 +914,29 @@ int enq_mechanics(hc_handle* h, bool forced, bool fuse = false, bool fuse_adv = 
   M.vv = vertex_view<T>(h);
   M.fuse_spread = 0;
   M.fuse_advance = 0;
+  M.after_prev = M.before_next = M.carveout = 0;
   M.tg = h->tg;
   // Fcur = the next step's force field; unode = this step's node velocities
   M.L = lbm_view<T>(h, h->cur, h->cur);
   M.f_limit = (T)h->u.f_limit;
-  if (h->p.launch == HC_LAUNCH_BATCHED && all_due && h->ncells > 0) {
+  const bool batched = h->p.launch == HC_LAUNCH_BATCHED && all_due && h->ncells > 0;
+  if (batched) {
     M.fuse_spread = fuse ? 1 : 0;
     M.fuse_advance = fuse && fuse_adv ? 1 : 0;
     if (M.fuse_advance) h->stamp_ahead = true;
+  }
+  if (batched && (h->tune[6] == 1 || (h->tune[6] == 0 && (used_types(h) > 1 || h->tune[5] > 0)))) {
+    // one launch across the cell types, largest first
     size_t smem = 0;
     for (TypeSlot& ts : h->types)
-      if (!ts.cells.empty()) smem = std::max(smem, mech_smem(h, ts, h->tune[6]));
+      if (!ts.cells.empty()) smem = std::max(smem, gather_bytes(h, ts));
     M.cells = h->dcells_all;
     M.ncells = h->ncells;
     M.dyn_smem = (int)smem;
-    HC_CUDA(h, hcd::launch_mechanics<T>(M, h->tune[4], h->tune[5], h->tune[6], h->stream));
+    HC_CUDA(h, hcd::launch_mechanics<T>(M, 1, h->tune[4], h->tune[5], h->tune[6], h->stream));
     return HC_OK;
   }
-  for (TypeSlot& ts : h->types) {
-    if (ts.cells.empty() || !(forced || h->iter % ts.every == 0)) continue;
-    M.cells = ts.dcells;
-    M.ncells = (int)ts.cells.size();
-    M.dyn_smem = (int)mech_smem(h, ts, h->tune[6]);
-    HC_CUDA(h, hcd::launch_mechanics<T>(M, h->tune[4], 0, h->tune[6], h->stream));
-  }
-  return HC_OK;
+  return enq_types<T>(h, M, forced, all_due);
 }
 
 // one HemoCell::iterate(): spread, collide+stream (+force reset), interpolate
@@ -1033,6 +1186,7 @@ int add_cells_positions(hc_handle* h, int type, int n, const std::vector<double>
   HC_CUDA(h, cudaStreamSynchronize(h->stream));
   h->nvert += n * nv;
   h->ncells += n;
+  apply_rules(h);
   if ((rc = ensure_repulsion(h)) != HC_OK) return rc;
   return upload_cell_lists(h);
 }
@@ -1086,6 +1240,7 @@ int autotune(hc_handle* h, const char* cache) {
         int old_tune[8];
         std::memcpy(old_tune, h->tune, sizeof(old_tune));
         std::memcpy(h->tune, t, sizeof(t));
+        h->tuned = true;
         if (!set_bulk_plan<T>(h, h->tune[7])) h->tune[7] = 0;
         invalidate_graph(h);
         return retag_if_needed(h, old_tune);
@@ -1183,6 +1338,7 @@ int autotune(hc_handle* h, const char* cache) {
   const int k1[][2] = {{0, 1},  {0, 2},  {0, 4},  {32, 4}, {64, 2}, {64, 4}, {128, 1}, {128, 2},
                        {256, 1}, {32, 8}, {8, 16}, {8, 32}, {16, 8}, {16, 16}};
   const int nvflags = h->tune[7] & 0x300;
+  h->tuned = true;
   float best = 1e30f;
   int bx = h->tune[0], by = h->tune[1], b7 = h->tune[7] & 0xff;
   auto try_k1 = [&](int x0, int y0, int code) {
@@ -1282,6 +1438,7 @@ int autotune(hc_handle* h, const char* cache) {
       for (int bs : {128, 256, 384, 512, 768})
         for (int gr : {0, 2 * sms}) {
           if (bs > (h->f64 ? 384 : 768)) continue;
+          if (var == 2 && (gr != 0 || bs > 384)) continue;  // a cluster per cell, at most 384 threads a CTA
           if (gr != 0 && h->p.launch != HC_LAUNCH_BATCHED) continue;
           h->tune[4] = bs;
           h->tune[5] = gr;
@@ -1500,6 +1657,7 @@ hc_handle* hc_create(const hc_params* p) {
   cudaMemsetAsync(h->bodyz, 0, 3 * h->ts * h->nz, h->stream);
   cudaMemsetAsync(h->status, 0, sizeof(unsigned int), h->stream);
   h->hflag.assign(h->N, 0);
+  cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, p->device);
   if (upload_flags(h) != HC_OK) return bail(h->err);
   if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return bail(cudaGetErrorString(e));
   return h;
@@ -1649,12 +1807,18 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
   const double mat[9] = {m->kLink, m->kBend, m->kVolume, m->kArea, m->eta_m,
                          m->kInnerRigid, m->kCytoskeleton, m->coreRadius, m->radius};
   ts.k = hcg::scale_material(model, nf, h->u, h->p.dx, h->p.dt, mat);
-  const size_t smem = (h->f64 ? hcd::mechanics_smem_bytes<double>(nv) : hcd::mechanics_smem_bytes<float>(nv));
+  const size_t smem = gather_bytes(h, ts);
   if (smem > 227 * 1024) return fail(h, HC_ERR_INVALID, "cell type too large for one CTA's shared memory");
+  HC_CUDA(h, h->f64 ? hcd::prepare_mechanics<double>((int)smem, &h->staged_limit)
+                    : hcd::prepare_mechanics<float>((int)smem, &h->staged_limit));
   {
-    size_t need = std::max(smem, mech_smem(h, ts, 2));
-    for (TypeSlot& o : h->types) need = std::max(need, std::max(mech_smem(h, o, 0), mech_smem(h, o, 2)));
-    HC_CUDA(h, h->f64 ? hcd::prepare_mechanics<double>((int)need) : hcd::prepare_mechanics<float>((int)need));
+    const size_t s16 = hcd::mechanics_staged_bytes(model, nv, nf, ts.tc.ne, 16, h->f64), g16 = gather_bytes(h, ts, 16);
+    ts.cluster16 =
+        s16 <= (size_t)h->staged_limit &&
+        (h->f64 ? hcd::mechanics_cluster_fits<double>(true, 16, 384, (int)s16) &&
+                      hcd::mechanics_cluster_fits<double>(false, 16, 384, (int)g16)
+                : hcd::mechanics_cluster_fits<float>(true, 16, 384, (int)s16) &&
+                      hcd::mechanics_cluster_fits<float>(false, 16, 384, (int)g16));
   }
   // one device blob: ints then doubles
   const hcg::TypeConstants& c = ts.tc;
@@ -1677,7 +1841,20 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
   };
   const size_t o_a0 = put_d(c.tri_a0), o_l0 = put_d(c.edge_l0), o_ang = put_d(c.edge_angle0),
                o_pd = put_d(c.patch_d0), o_il = put_d(c.inner_l0), o_sa = put_d(c.slot_a0), o_sl = put_d(c.slot_l0);
-  std::vector<float> fv(dv.begin(), dv.end());
+  // the mixed form reads 32-bit copies, the plain form the reciprocals of the
+  // rest areas and lengths
+  std::vector<float> fv;
+  size_t o_ia = 0, o_iel = 0;
+  if (h->f64) {
+    auto reciprocals = [](std::vector<double> a) {
+      for (double& x : a) x = 1.0 / x;
+      return a;
+    };
+    o_ia = put_d(reciprocals(c.tri_a0));
+    o_iel = put_d(reciprocals(c.edge_l0));
+  } else {
+    fv.assign(dv.begin(), dv.end());
+  }
   const size_t ib = 4 * iv.size(), db = 8 * std::max<size_t>(dv.size(), 1), fb = 4 * std::max<size_t>(fv.size(), 1);
   HC_CUDA(h, dalloc(h, &ts.blob, ib + db + fb));
   HC_CUDA(h, cudaMemcpyAsync(ts.blob, iv.data(), ib, cudaMemcpyHostToDevice, h->stream));
@@ -1714,6 +1891,8 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
   d.slot_l0f = fbase + o_sl;
   d.tri_a0 = dbase + o_a0;
   d.edge_l0 = dbase + o_l0;
+  d.tri_ia0 = h->f64 ? dbase + o_ia : nullptr;
+  d.edge_il0 = h->f64 ? dbase + o_iel : nullptr;
   d.edge_angle0 = dbase + o_ang;
   d.patch_d0 = dbase + o_pd;
   d.inner_l0 = dbase + o_il;
@@ -2288,6 +2467,7 @@ int hc_set_tuning(hc_handle* h, const int* in8) {
   int old_tune[8];
   std::memcpy(old_tune, h->tune, sizeof(old_tune));
   std::memcpy(h->tune, in8, sizeof(h->tune));
+  h->tuned = true;
   invalidate_graph(h);
   return retag_if_needed(h, old_tune);
 }

@@ -13,6 +13,7 @@
 
 #include "hc_async.cuh"
 #include "hc_d3q19.cuh"
+#include "hc_newton.h"
 #include "hc_posbits.h"
 
 namespace hcd {
@@ -21,6 +22,15 @@ template <typename T>
 __device__ __forceinline__ T tmax(T a, T b) {
   return a > b ? a : b;
 }
+
+// x == 0 and isfinite(x) on the bits of a double: a comparison would take an
+// instruction of the FP64 pipe
+__device__ __forceinline__ bool is_zero(float x) { return x == 0.f; }
+__device__ __forceinline__ bool is_zero(double x) {
+  return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
+}
+__device__ __forceinline__ bool is_finite(float x) { return isfinite(x); }
+__device__ __forceinline__ bool is_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 
 // IBM phi2 kernel (core/immersedBoundaryMethod.h:37-41, :62-138).  The
 // reference scans the 3x3x3 nodes around floor(p+0.5) and keeps the nonzero
@@ -48,10 +58,22 @@ __device__ __forceinline__ void ibm_weights(const LbmView<T>& L, double px, doub
   for (int a = 0; a < 3; ++a) {
     long long qi;
     if (kF64) {
-      const double q0 = floor(P[a]);
-      phi[a][0] = tmax(T(1) - T(fabs(P[a] - q0)), T(0));
-      phi[a][1] = tmax(T(1) - T(fabs(P[a] - (q0 + 1.0))), T(0));
-      qi = (long long)q0;
+      // floor(P) from the bits of P as well: P - floor(P) is then the one FP64
+      // instruction, and both weights are the bits of the expression below it
+      // (1 - |P - (q + 1)| is exactly the fraction for P >= 1)
+      int qs;
+      double q0;
+      if (hcpos::floor_bits(P[a], qs, q0)) {
+        const T fr = T(P[a] - q0);
+        phi[a][0] = T(1) - fr;
+        phi[a][1] = fr;
+        qi = qs;
+      } else {
+        q0 = floor(P[a]);
+        phi[a][0] = tmax(T(1) - T(fabs(P[a] - q0)), T(0));
+        phi[a][1] = tmax(T(1) - T(fabs(P[a] - (q0 + 1.0))), T(0));
+        qi = (long long)q0;
+      }
     } else {
       // floor(P) and the fraction (float)(P - floor(P)) from the bits of P,
       // the FP64 instructions only outside [1, 2^31)
@@ -91,19 +113,33 @@ __device__ __forceinline__ void ibm_weights(const LbmView<T>& L, double px, doub
     }
   }
   T total = T(0);
+  bool cut = false;  // a node that carries weight was left out
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
     const int ax = s >> 2, ay = (s >> 1) & 1, az = s & 1;
     K.node[s] = -1;
     K.w[s] = T(0);
-    if (idx[0][ax] < 0 || idx[1][ay] < 0 || idx[2][az] < 0) continue;
+    if (idx[0][ax] < 0 || idx[1][ay] < 0 || idx[2][az] < 0) {
+      cut = true;
+      continue;
+    }
     const T w = phi[0][ax] * phi[1][ay] * phi[2][az];
-    if (w == T(0)) continue;
+    if (is_zero(w)) continue;
     const int nd = idx[0][ax] + L.nx * (idx[1][ay] + L.ny * idx[2][az]);
-    if (!HC_IN(L.status, nd, L.N) || L.flag[nd] != 0) continue;
-    total += w;
+    if (!HC_IN(L.status, nd, L.N) || L.flag[nd] != 0) {
+      cut = true;
+      continue;
+    }
+    if (!kF64) total += w;
     K.node[s] = nd;
     K.w[s] = w;
+  }
+  // The weights of a whole stencil sum to one by themselves, to the rounding
+  // of their products: FP64, whose pipe bounds the cell kernels, renormalises
+  // only a stencil that lost a node (24 of its 60 instructions otherwise).
+  if (kF64 && cut) {
+#pragma unroll
+    for (int s = 0; s < 8; ++s) total += K.w[s];
   }
   if (total > T(0)) {
     const T coeff = T(1) / total;
@@ -461,7 +497,7 @@ __global__ void __launch_bounds__(256) k_interp_advance(const LbmView<T> L, cons
     vv.v[i] = vx;
     vv.v[V + i] = vy;
     vv.v[2 * V + i] = vz;
-    if (!(isfinite(vx) && isfinite(vy) && isfinite(vz))) atomicOr(vv.status, 1u);
+    if (!(is_finite(vx) && is_finite(vy) && is_finite(vz))) atomicOr(vv.status, 1u);
   } else {
     vx = vv.v[i];
     vy = vv.v[V + i];
@@ -603,6 +639,11 @@ __device__ __forceinline__ float third<float>(float a) {
 template <typename T>
 __device__ __forceinline__ V3t<T> unit_normal(V3t<T> a, V3t<T> b, V3t<T> c) {
   V3t<T> n = vcross(b - a, c - a);
+  if constexpr (sizeof(T) == 8) {
+    T inv, len;
+    hcnewton::inv_length(vdot(n, n), inv, len);
+    return vscale(n, inv);
+  }
   const T l = vnorm(n);
   if (l != T(0)) return {n.x / l, n.y / l, n.z / l};
   return {T(0), T(0), T(0)};
@@ -635,12 +676,54 @@ __device__ __forceinline__ float rest_value<float>(const double*, const float* f
   return f[k];
 }
 
-template <typename T>
-size_t mechanics_smem_bytes(int nv) {
-  return 34 * sizeof(double) + 6 * (size_t)nv * sizeof(T) + (size_t)nv;
+// Cells on clusters of CTAs: rank r of a cluster owns a run of whole warps of
+// the cell's vertices (and faces, edges): items [r c, (r + 1) c) with
+// c = cluster_chunk(n, cluster size).
+__host__ __device__ __forceinline__ int cluster_chunk(int n, int cluster) {
+  return ((n + cluster - 1) / cluster + 31) / 32 * 32;
 }
+constexpr int kClusterHeader = 40;
+template <typename T>
+size_t mechanics_smem_bytes(int nv, int cluster) {
+  return kClusterHeader * sizeof(double) + (3 * (size_t)nv + 3 * (size_t)cluster_chunk(nv, cluster)) * sizeof(T) +
+         (size_t)nv;
+}
+template <typename T>
+__device__ __forceinline__ V3t<T> ld3_cluster(uint32_t a) {
+  V3t<T> v;
+  ld_cluster(a, v.x);
+  ld_cluster(a + (uint32_t)sizeof(T), v.y);
+  ld_cluster(a + 2u * (uint32_t)sizeof(T), v.z);
+  return v;
+}
+// the sum of a double over the ranks, in their order: the same bits in each
+__device__ __forceinline__ double cluster_sum(const double* p, int cs) {
+  double sum = 0.0;
+  for (int r = 0; r < cs; ++r) {
+    double part;
+    ld_cluster(cluster_addr(smem_addr(p), (uint32_t)r), part);
+    sum += part;
+  }
+  return sum;
+}
+// Where item k of an array cut into chunks lies: its address in the owner's
+// shared memory.  magic = ceil(2^32 / chunk) makes the division exact for
+// k * chunk < 2^32 (at most 19,000 faces in chunks of at most that many).
+struct Chunked {
+  uint32_t base, stride, magic;
+  int chunk;
+  __device__ __forceinline__ Chunked(const void* p, int chunk_, size_t stride_)
+      : base(smem_addr(p)), stride((uint32_t)stride_), magic((uint32_t)((0x100000000ull + chunk_ - 1) / chunk_)),
+        chunk(chunk_) {}
+  __device__ __forceinline__ uint32_t owner(int k) const { return __umulhi((uint32_t)k, magic); }
+  __device__ __forceinline__ uint32_t within(int k, uint32_t own) const { return (uint32_t)k - own * (uint32_t)chunk; }
+  __device__ __forceinline__ uint32_t at(int k, uint32_t own) const {
+    return cluster_addr(base + within(k, own) * stride, own);
+  }
+  __device__ __forceinline__ uint32_t at(int k) const { return at(k, owner(k)); }
+};
 
-// One CTA per cell (grid-stride over the cell list), vertex-centric: each
+// One CTA or cluster per cell (grid-stride over the cell list), vertex-centric: each
 // thread owns vertices and sums, in a fixed order, every contribution the
 // reference's face / edge / vertex loops deposit on them
 // (rbcHighOrderModel.cpp:56-204, pltSimpleModel.cpp:59-205,
@@ -682,8 +765,15 @@ template <typename T>
 __device__ __forceinline__ V3t<T> plt_bending(const T* sx, const TypeDev& t, int e) {
   const int a = t.edges[2 * e], b = t.edges[2 * e + 1];
   const V3t<T> ev = ld3(sx, b) - ld3(sx, a);
-  const T L = vnorm(ev);
-  const V3t<T> uv = {ev.x / L, ev.y / L, ev.z / L};
+  V3t<T> uv;
+  if constexpr (sizeof(T) == 8) {
+    T inv, len;
+    hcnewton::inv_length(vdot(ev, ev), inv, len);
+    uv = vscale(ev, inv);
+  } else {
+    const T L = vnorm(ev);
+    uv = {ev.x / L, ev.y / L, ev.z / L};
+  }
   const int* A = t.tris + 3 * t.bend_tris[2 * e];
   const int* B = t.tris + 3 * t.bend_tris[2 * e + 1];
   const V3t<T> V1 = unit_normal(ld3(sx, A[0]), ld3(sx, A[1]), ld3(sx, A[2]));
@@ -706,8 +796,11 @@ __device__ __forceinline__ void spread_vertex(const MechView<T>& M, int gi, V3t<
   T mag = f.x * f.x;
   mag += f.y * f.y;
   mag += f.z * f.z;
-  mag = sqrt(mag);
-  if (mag > M.f_limit) f = vscale(f, M.f_limit / mag);
+  // the FP64 square root (ten FP64 instructions) only near or above the limit
+  if (sizeof(T) == 4 || mag > T(0.999999) * M.f_limit * M.f_limit) {
+    mag = sqrt(mag);
+    if (mag > M.f_limit) f = vscale(f, M.f_limit / mag);
+  }
   if (vv.frep_cell) f = f + V3t<T>{vv.frep_cell[gi], vv.frep_cell[V + gi], vv.frep_cell[2 * V + gi]};
   if (vv.frep_wall) f = f + V3t<T>{vv.frep_wall[gi], vv.frep_wall[V + gi], vv.frep_wall[2 * V + gi]};
   Kern<T> K;
@@ -732,13 +825,13 @@ __device__ __forceinline__ void spread_vertex(const MechView<T>& M, int gi, V3t<
 // `hit` is a shared flag the caller cleared before its last barrier.  Returns
 // whether the cell is still alive; the deletion is written to the cell's state
 // by thread 0.  Ends with a barrier: every vertex is advanced and binned.
+// advance_range does vertices [k0, k1) of the cell, without the barrier.
 template <typename T>
-__device__ __forceinline__ bool advance_cell(const MechView<T>& M, const TypeDev& t, int cell, int voff, bool alive,
-                                             int& hit) {
+__device__ __forceinline__ void advance_range(const MechView<T>& M, int voff, int k0, int k1, bool alive, int& hit) {
   const VertexView<T>& vv = M.vv;
   const LbmView<T>& L = M.L;
   const long long V = vv.V;
-  for (int k = threadIdx.x; k < t.nv; k += blockDim.x) {
+  for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
     const int i = voff + k;
     if (!alive) {
       vv.vnode[i] = -1;
@@ -761,7 +854,7 @@ __device__ __forceinline__ bool advance_cell(const MechView<T>& M, const TypeDev
     vv.v[i] = vx;
     vv.v[V + i] = vy;
     vv.v[2 * V + i] = vz;
-    if (!(isfinite(vx) && isfinite(vy) && isfinite(vz))) atomicOr(vv.status, STATUS_NONFINITE);
+    if (!(is_finite(vx) && is_finite(vy) && is_finite(vz))) atomicOr(vv.status, STATUS_NONFINITE);
     px += (double)vx;
     py += (double)vy;
     pz += (double)vz;
@@ -794,29 +887,25 @@ __device__ __forceinline__ bool advance_cell(const MechView<T>& M, const TypeDev
     vv.vtile[i] = q[0] / M.tg.tx + M.tg.ntx * (q[1] / M.tg.ty + M.tg.nty * (q[2] / M.tg.tz));
     if (L.flag[nd] != 0) hit = 1;
   }
-  __syncthreads();
-  const bool deleted = alive && hit;
-  if (threadIdx.x == 0 && deleted) {
-    vv.alive[cell] = 0;
-    atomicOr(vv.status, STATUS_CELL_DELETED);
-  }
-  return alive && !deleted;
 }
-
-// The vertex-centric force assembly of one cell (variant 0; the staged
-// variant falls back to it for cell types too large for its shared memory).
-// sx holds 6 nv T + nv bytes of shared memory after `red` (34 doubles).
+// The vertex-centric force assembly of one cell's vertices [v0, v1) and faces
+// [f0, f1) by one rank of its cluster (variant 0; the staged variant falls back
+// to it for FP32 cell types whose terms would not share an SM).  sx holds
+// 3 nv T, the own bending forces and nv bytes of shared memory after `red`.
+// Every rank of the cluster calls it: it holds the cluster's barriers.
 template <typename T>
-__device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev& t, int voff, bool alive, double* red,
-                                            T* sx) {
+__device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev& t, int voff, bool alive, int cs,
+                                            int rank, double* red, T* sx) {
   const VertexView<T>& vv = M.vv;
   const long long V = vv.V;
   const int tid = threadIdx.x, bs = blockDim.x;
   constexpr bool kF64 = sizeof(T) == 8;
-  const int nv = t.nv;
-  T* sbf = sx + 3 * nv;  // own bending force per vertex
-  uint8_t* srn = reinterpret_cast<uint8_t*>(sbf + 3 * nv);  // valence per vertex
-  if (!HC_IN(vv.status, (long long)voff + nv - 1, V)) return;  // the cell's vertices in the arrays
+  const int nv = t.nv, vch = cluster_chunk(nv, cs), fch = cluster_chunk(t.nf, cs);
+  const int v0 = min(rank * vch, nv), v1 = min(v0 + vch, nv);
+  const int f0 = min(rank * fch, t.nf), f1 = min(f0 + fch, t.nf);
+  T* sbf = sx + 3 * nv;  // own bending force per own vertex
+  uint8_t* srn = reinterpret_cast<uint8_t*>(sbf + 3 * vch);  // valence per vertex
+  if (!HC_IN(vv.status, (long long)voff + nv - 1, V)) return;  // the cell's vertices in the arrays (every rank returns)
   for (int k = tid; k < nv; k += bs) srn[k] = (uint8_t)t.ring_n[k];
   // positions relative to the cell's vertex 0 (translation invariant forces;
   // the volume sum stays well conditioned far from the origin)
@@ -828,7 +917,7 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
   }
   __syncthreads();
   if (!alive) {
-    for (int k = tid; k < nv; k += bs) {
+    for (int k = v0 + tid; k < v1; k += bs) {
       vv.f[voff + k] = T(0);
       vv.f[V + voff + k] = T(0);
       vv.f[2 * V + voff + k] = T(0);
@@ -837,7 +926,7 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
   }
   // --- phase 1: face volume terms, own bending force (rbcHighOrderModel.cpp:62-68, :127-157)
   double vol = 0.0;
-  for (int k = tid; k < t.nf; k += bs) {
+  for (int k = f0 + tid; k < f1; k += bs) {
     const V3t<T> v0 = ld3(sx, t.tris[3 * k]), v1 = ld3(sx, t.tris[3 * k + 1]), v2 = ld3(sx, t.tris[3 * k + 2]);
     if (kF64) {
       const double v210 = (double)v2.x * v1.y * v0.z, v120 = (double)v1.x * v2.y * v0.z;
@@ -850,7 +939,7 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
     }
   }
   if (t.model != 1) {
-    for (int i = tid; i < nv; i += bs) {
+    for (int i = v0 + tid; i < v1; i += bs) {
       const int rn = t.ring_n[i];
       const int* rg = t.ring + 6 * i;
       const V3t<T> xi = ld3(sx, i);
@@ -872,15 +961,18 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
       const T ndev = vdot(pn, dev);
       const T dDev = fdiv(ndev - rest_value<T>(t.patch_d0, t.patch_d0f, i), (T)t.edge_mean_eq);
       const V3t<T> bf = vscale(pn, (T)t.k_bend * (dDev + fdiv(dDev, fabs(T(kMaxBend) - dDev * dDev))));
-      sbf[3 * i] = bf.x;
-      sbf[3 * i + 1] = bf.y;
-      sbf[3 * i + 2] = bf.z;
+      T* q = sbf + 3 * (i - v0);
+      q[0] = bf.x;
+      q[1] = bf.y;
+      q[2] = bf.z;
     }
   }
-  block_sum<T>(vol, red);  // red[32] = sum over the block (synchronises)
+  block_sum<T>(vol, red);  // red[32] = sum over the block
+  cluster_sync(cs);
+  const Chunked bending(sbf, vch, 3 * sizeof(T));
   // volume constraint in FP64 (rbcHighOrderModel.cpp:100-104), by one thread
   if (tid == 0) {
-    const double volume = red[32] * (1.0 / 6.0);
+    const double volume = cluster_sum(red + 32, cs) * (1.0 / 6.0);
     const double vfr = (volume - t.volume_eq) / t.volume_eq;
     const double vf = -t.k_volume * vfr / fabs(kMaxVol - vfr * vfr);
     red[33] = vf;
@@ -892,7 +984,7 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
   const T area_mean = (T)t.area_mean_eq;
   const bool visc = (t.model != 0) || (t.eta_m != 0.0);
   // --- phase 2: gather per vertex
-  for (int i = tid; i < nv; i += bs) {
+  for (int i = v0 + tid; i < v1; i += bs) {
     const int rn = t.ring_n[i];
     const V3t<T> xi = ld3(sx, i);
     V3t<T> f = {T(0), T(0), T(0)};
@@ -956,14 +1048,15 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
       if (t.model != 1) {
         // neighbour's bending reaction -bf_r / n_r
         const T rnr = (T)srn[r];
-        f = f + V3t<T>{fdiv(-sbf[3 * r], rnr), fdiv(-sbf[3 * r + 1], rnr), fdiv(-sbf[3 * r + 2], rnr)};
+        const V3t<T> b = ld3_cluster<T>(bending.at(r));
+        f = f + V3t<T>{fdiv(-b.x, rnr), fdiv(-b.y, rnr), fdiv(-b.z, rnr)};
       } else {
         // platelet dihedral terms: end point of edge e, outer point of the opposite edge
         f = f + plt_bending(sx, t, e);
         f = f - plt_bending(sx, t, t.vopp[6 * i + j]);
       }
     }
-    if (t.model != 1) f = f + ld3(sbf, i);
+    if (t.model != 1) f = f + ld3(sbf, i - v0);
     // inner links (pltSimpleModel.cpp:188-205, wbcHighOrderModel.cpp:202-223)
     for (int q = t.vinner_off[i]; q < t.vinner_off[i + 1]; ++q) {
       const int e = t.vinner[q];
@@ -987,232 +1080,306 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
   }
 }
 
+// The start of a cell's assembly, by every rank of its cluster: the type record
+// into shared memory (set-up data, read before the programmatic wait), then with
+// fuse_advance the interpolation and advance of the rank's vertices.  Returns
+// whether the cell is alive; with fuse_advance the ranks are synchronised and
+// every vertex is advanced.
 template <typename T>
-__global__ void __launch_bounds__(sizeof(T) == 8 ? 384 : 768) k_mechanics(const MechView<T> M) {
-  pdl_wait();
-  extern __shared__ double smem_d[];
-  __shared__ TypeDev tshared;
-  double* red = smem_d;  // 34 doubles
-  T* sx = reinterpret_cast<T*>(smem_d + 34);
-  __shared__ int hit;
-  for (int ci = blockIdx.x; ci < M.ncells; ci += gridDim.x) {
-    const int cell = M.cells[ci];
-    __syncthreads();  // previous cell fully written out
-    if (threadIdx.x == 0) {
-      tshared = M.types[M.cell_type[cell]];
-      hit = 0;
-    }
-    // the cell's scalars load while thread 0 fetches the type
-    const int voff = M.cell_voff[cell];
-    bool alive = M.vv.alive[cell] != 0;
-    __syncthreads();
-    if (M.fuse_advance) alive = advance_cell(M, tshared, cell, voff, alive, hit);
-    gather_cell(M, tshared, voff, alive, red, sx);
+__device__ __forceinline__ bool begin_cell(const MechView<T>& M, int cell, int voff, int cs, int rank, TypeDev& t,
+                                           int& hit) {
+  const VertexView<T>& vv = M.vv;
+  const int tid = threadIdx.x, lane = tid & 31;
+  static_assert(sizeof(TypeDev) % 8 == 0, "copied in 8-byte words");
+  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(M.types + M.cell_type[cell]);
+  for (int w = tid; w < (int)(sizeof(TypeDev) / 8); w += blockDim.x)
+    reinterpret_cast<unsigned long long*>(&t)[w] = src[w];
+  if (tid == 0) hit = 0;
+  // Behind another type's launch: that one let this start after its own wait
+  // for everything before it, and this one reads nothing that it writes.
+  if (!M.after_prev) pdl_wait();
+  if (M.before_next) pdl_trigger();
+  bool alive = vv.alive[cell] != 0;
+  __syncthreads();
+  if (!M.fuse_advance) return alive;
+  const int nv = t.nv, vch = cluster_chunk(nv, cs), v0 = min(rank * vch, nv);
+  advance_range(M, voff, v0, min(v0 + vch, nv), alive, hit);
+  cluster_sync(cs);
+  // the ranks' flags together; rank 0 writes the cell's state, which every rank
+  // read before the barrier
+  int h = 0;
+  for (int r = lane; r < cs; r += 32) h |= ld_cluster_int(cluster_addr(smem_addr(&hit), (uint32_t)r));
+  const bool deleted = alive && __any_sync(0xffffffffu, h != 0);
+  if (deleted && rank == 0 && tid == 0) {
+    vv.alive[cell] = 0;
+    atomicOr(vv.status, STATUS_CELL_DELETED);
   }
+  return alive && !deleted;
+}
+
+// The end of a launch: the next kernel waits for this one alone, so this one may
+// not end before the type's launch before it.
+template <typename T>
+__device__ __forceinline__ void end_launch(const MechView<T>& M) {
+  if (M.after_prev && blockIdx.x == 0) pdl_wait();
   pdl_trigger();
 }
 
-// Staged variant (2): every face's area-force scalar, centroid and
-// area-weighted normal, and every edge's link force (with membrane viscosity
-// and the platelet dihedral force) are computed once into shared memory;
-// each vertex then gathers the terms of its incident faces and edges, its own
-// and its neighbours' bending, and its inner links.  Deterministic like the
-// vertex-centric variant, which computes each face and edge once per
-// incident vertex; a cell type whose terms do not fit the launch's shared
-// memory takes that variant's path.  Shared layout after `red` (34 doubles):
-// positions 3 nv, own bending 3 nv, faces 7 nf (centroid, area-force scalar,
-// area x unit normal), edges 3 ne (force on the lower-numbered end), platelet
-// dihedral 3 ne (platelets only), valence nv bytes.
 template <typename T>
-__host__ __device__ __forceinline__ size_t staged_smem_bytes(int model, int nv, int nf, int ne) {
-  const size_t words = 6 * (size_t)nv + 7 * (size_t)nf + 3 * (size_t)ne * (model == 1 ? 2 : 1);
-  return 34 * sizeof(double) + words * sizeof(T) + (size_t)nv;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(sizeof(T) == 8 ? 384 : 768) k_mechanics_staged(const MechView<T> M) {
-  pdl_wait();
+__global__ void __launch_bounds__(sizeof(T) == 8 ? 384 : 768) k_mechanics(const MechView<T> M) {
   extern __shared__ double smem_d[];
   __shared__ TypeDev tshared;
-  double* red = smem_d;
-  T* sx = reinterpret_cast<T*>(smem_d + 34);
+  __shared__ int hit;
+  const int cs = (int)cluster_size(), rank = (int)cluster_rank();
+  for (int ci = blockIdx.x / cs; ci < M.ncells; ci += gridDim.x / cs) {
+    const int cell = M.cells[ci], voff = M.cell_voff[cell];
+    const bool alive = begin_cell(M, cell, voff, cs, rank, tshared, hit);
+    gather_cell(M, tshared, voff, alive, cs, rank, smem_d, reinterpret_cast<T*>(smem_d + kClusterHeader));
+    cluster_sync(cs);  // no rank goes on or leaves while another reads its terms
+  }
+  end_launch(M);
+}
+
+// Staged variant (2): each cell on a cluster of 1 to 16 CTAs.  Rank r of the
+// cluster owns a run of whole warps of the cell's vertices, faces and edges; it
+// interpolates and advances its vertices, computes its faces' and edges' terms
+// once into its own shared memory and gathers the forces of its vertices,
+// reading the terms of other ranks through distributed shared memory.  Every
+// rank holds all positions of the cell.
+//
+// What bounds it: in FP64 the FP64 pipe (two lanes an SM and cycle).  One CTA
+// per cell left that pipe idle on every SM without a cell, and on all but one
+// SM of a one-cell run; a vertex cost about 2100 FP64 instructions.  Here each
+// face and edge is computed once, normalisation takes one reciprocal square
+// root, saturation terms one reciprocal, the face's volume force is its cross
+// product (area times unit normal), bending normals are the faces' and rest
+// values come as reciprocals.  Area and link forces (and the membrane
+// viscosity) act along the edges: a face gives each corner a third of its area
+// scalar along both of the corner's edges, so a vertex needs one scalar per
+// face and one per edge instead of two vectors.
+//
+// Shared layout after a header of 40 doubles: faces 4 words (cross product,
+// area scalar) and 1 word (inverse length of the cross product) of the own
+// chunk, positions 3 nv, own bending 3 vch, edge scalars ech, platelet dihedral
+// 3 ech (platelets only), valence nv bytes.
+template <typename T>
+__host__ __device__ __forceinline__ size_t staged_smem_bytes(int model, int nv, int nf, int ne, int cluster) {
+  const size_t words = 5 * (size_t)cluster_chunk(nf, cluster) + 3 * (size_t)nv + 3 * (size_t)cluster_chunk(nv, cluster) +
+                       (size_t)cluster_chunk(ne, cluster) * (model == 1 ? 4 : 1);
+  return kClusterHeader * sizeof(double) + words * sizeof(T) + (size_t)nv;
+}
+
+// x + x / |limit - x^2|, the saturating response of every membrane term
+__device__ __forceinline__ float saturating(float x, float limit) { return x + fdiv(x, fabsf(limit - x * x)); }
+__device__ __forceinline__ double saturating(double x, double limit) {
+  return fma(x, hcnewton::recip(fabs(fma(-x, x, limit))), x);
+}
+// (value - rest) / rest
+__device__ __forceinline__ float strain(float v, const double*, const float* rest, const double*, int k) {
+  const float r = rest[k];
+  return fdiv(v - r, r);
+}
+__device__ __forceinline__ double strain(double v, const double* rest, const float*, const double* inv, int k) {
+  return (v - rest[k]) * inv[k];
+}
+// 1 / n for a valence of 3 to 6
+template <typename T>
+__device__ __forceinline__ T inv_valence(int n) {
+  return n == 6 ? T(1.0 / 6.0) : (n == 5 ? T(0.2) : (n == 4 ? T(0.25) : T(1.0 / 3.0)));
+}
+// a / b by a reciprocal: fast in both forms
+__device__ __forceinline__ float quotient(float a, float b) { return fdiv(a, b); }
+__device__ __forceinline__ double quotient(double a, double b) { return a * hcnewton::recip(b); }
+template <typename T>
+__global__ void __launch_bounds__(384) k_mechanics_staged(const MechView<T> M) {
+  extern __shared__ __align__(16) double smem_cluster[];
+  __shared__ TypeDev t;
+  __shared__ int hit;
+  const int tid = threadIdx.x, bs = blockDim.x;
+  const int cs = (int)cluster_size(), rank = (int)cluster_rank();
   const VertexView<T>& vv = M.vv;
   const long long V = vv.V;
-  const int tid = threadIdx.x, bs = blockDim.x;
-  constexpr bool kF64 = sizeof(T) == 8;
-  __shared__ int hit;
-  for (int ci = blockIdx.x; ci < M.ncells; ci += gridDim.x) {
-    const int cell = M.cells[ci];
-    __syncthreads();
-    if (tid == 0) {
-      tshared = M.types[M.cell_type[cell]];
-      hit = 0;
+  const int cell = M.cells[blockIdx.x / cs], voff = M.cell_voff[cell];
+  bool alive = begin_cell(M, cell, voff, cs, rank, t, hit);
+  const int nv = t.nv, nf = t.nf, ne = t.ne;
+  const bool plt = t.model == 1, visc = (t.model != 0) || (t.eta_m != 0.0);
+  const int vch = cluster_chunk(nv, cs), fch = cluster_chunk(nf, cs), ech = cluster_chunk(ne, cs);
+  const int v0 = min(rank * vch, nv), v1 = min(v0 + vch, nv);
+  const int f0 = min(rank * fch, nf), f1 = min(f0 + fch, nf);
+  const int e0 = min(rank * ech, ne), e1 = min(e0 + ech, ne);
+  double* red = smem_cluster;
+  T* sface = reinterpret_cast<T*>(smem_cluster + kClusterHeader);
+  T* sinv = sface + 4 * fch;
+  T* sx = sinv + fch;
+  T* sbf = sx + 3 * nv;
+  T* sedge = sbf + 3 * vch;
+  T* splt = sedge + ech;
+  uint8_t* srn = reinterpret_cast<uint8_t*>(splt + (plt ? 3 * ech : 0));
+  if (!HC_IN(vv.status, (long long)voff + nv - 1, V)) alive = false;
+  if (!alive) {
+    for (int k = v0 + tid; k < v1; k += bs) {
+      if (!HC_IN(vv.status, voff + k, V)) break;
+      vv.f[voff + k] = T(0);
+      vv.f[V + voff + k] = T(0);
+      vv.f[2 * V + voff + k] = T(0);
     }
-    const int voff = M.cell_voff[cell];
-    bool alive = vv.alive[cell] != 0;
-    __syncthreads();
-    const TypeDev& t = tshared;
-    if (M.fuse_advance) alive = advance_cell(M, t, cell, voff, alive, hit);
-    if (staged_smem_bytes<T>(t.model, t.nv, t.nf, t.ne) > (size_t)M.dyn_smem) {
-      gather_cell(M, t, voff, alive, red, sx);
-      continue;
+    cluster_sync(cs);  // no rank leaves while another may still read its flag
+    end_launch(M);
+    return;
+  }
+  // positions relative to the cell's vertex 0
+  const double r0x = vv.x[voff], r0y = vv.x[V + voff], r0z = vv.x[2 * V + voff];
+  for (int k = tid; k < nv; k += bs) {
+    srn[k] = (uint8_t)t.ring_n[k];
+    sx[3 * k] = (T)(vv.x[voff + k] - r0x);
+    sx[3 * k + 1] = (T)(vv.x[V + voff + k] - r0y);
+    sx[3 * k + 2] = (T)(vv.x[2 * V + voff + k] - r0z);
+  }
+  __syncthreads();
+  // --- own faces: six times the signed volume, area force, cross product
+  double vol = 0.0;
+  for (int k = f0 + tid; k < f1; k += bs) {
+    const V3t<T> a = ld3(sx, t.tris[3 * k]), b = ld3(sx, t.tris[3 * k + 1]), c = ld3(sx, t.tris[3 * k + 2]);
+    const V3t<T> n = vcross(b - a, c - a);
+    vol += (double)vdot(a, n);
+    T inv, len;
+    hcnewton::inv_length(vdot(n, n), inv, len);
+    const T ar = strain(T(0.5) * len, t.tri_a0, t.tri_a0f, t.tri_ia0, k);
+    T* q = sface + 4 * (k - f0);
+    q[0] = n.x;
+    q[1] = n.y;
+    q[2] = n.z;
+    q[3] = (T)t.k_area * saturating(ar, T(kMaxArea));
+    sinv[k - f0] = inv;
+  }
+  // --- own edges: link and viscous force per edge vector, dihedral force
+  for (int e = e0 + tid; e < e1; e += bs) {
+    const int a = t.edges[2 * e], b = t.edges[2 * e + 1];
+    const V3t<T> d = ld3(sx, b) - ld3(sx, a);
+    T inv, len;
+    hcnewton::inv_length(vdot(d, d), inv, len);
+    const T ef = strain(len, t.edge_l0, t.edge_l0f, t.edge_il0, e);
+    T pull = (T)t.k_link * saturating(ef, T(kMaxLink));
+    if (visc) {
+      const V3t<T> va = {vv.v[voff + a], vv.v[V + voff + a], vv.v[2 * V + voff + a]};
+      const V3t<T> vb = {vv.v[voff + b], vv.v[V + voff + b], vv.v[2 * V + voff + b]};
+      const T fv = vdot(vb - va, d) * inv * (T)t.eta_m;
+      const T lim = T(kForceLimit / 4.0);
+      pull += fv > lim ? lim : (fv < -lim ? -lim : fv);
     }
-    const int nv = t.nv, nf = t.nf, ne = t.ne;
-    const bool plt = t.model == 1;
-    T* sbf = sx + 3 * nv;
-    T* sface = sbf + 3 * nv;
-    T* sedge = sface + 7 * nf;
-    T* spltb = sedge + 3 * ne;
-    uint8_t* srn = reinterpret_cast<uint8_t*>(spltb + (plt ? 3 * ne : 0));
-    const double r0x = vv.x[voff], r0y = vv.x[V + voff], r0z = vv.x[2 * V + voff];
-    for (int k = tid; k < nv; k += bs) {
-      srn[k] = (uint8_t)t.ring_n[k];
-      sx[3 * k] = (T)(vv.x[voff + k] - r0x);
-      sx[3 * k + 1] = (T)(vv.x[V + voff + k] - r0y);
-      sx[3 * k + 2] = (T)(vv.x[2 * V + voff + k] - r0z);
+    sedge[e - e0] = pull * inv;
+    if (plt) {
+      const V3t<T> pb = plt_bending(sx, t, e);
+      T* p = splt + 3 * (e - e0);
+      p[0] = pb.x;
+      p[1] = pb.y;
+      p[2] = pb.z;
     }
-    __syncthreads();
-    if (!alive) {
-      for (int k = tid; k < nv; k += bs) {
-        vv.f[voff + k] = T(0);
-        vv.f[V + voff + k] = T(0);
-        vv.f[2 * V + voff + k] = T(0);
-      }
-      continue;
-    }
-    const bool visc = (t.model != 0) || (t.eta_m != 0.0);
-    // --- phase A: faces, edges and bending, each once
-    double vol = 0.0;
-    for (int k = tid; k < nf; k += bs) {
-      const V3t<T> v0 = ld3(sx, t.tris[3 * k]), v1 = ld3(sx, t.tris[3 * k + 1]), v2 = ld3(sx, t.tris[3 * k + 2]);
-      const V3t<T> c = vcross(v1 - v0, v2 - v0);
-      if (kF64) {
-        const double v210 = (double)v2.x * v1.y * v0.z, v120 = (double)v1.x * v2.y * v0.z;
-        const double v201 = (double)v2.x * v0.y * v1.z, v021 = (double)v0.x * v2.y * v1.z;
-        const double v102 = (double)v1.x * v0.y * v2.z, v012 = (double)v0.x * v1.y * v2.z;
-        vol += (-v210 + v120 + v201 - v021 - v102 + v012);
-      } else {
-        vol += (double)vdot(v0, c);
-      }
-      T nn;
-      const V3t<T> n = normalized(c, nn);
-      const T area = nn != T(0) ? T(0.5) * nn : T(0);
-      const V3t<T> na = nn != T(0) ? vscale(n, area) : V3t<T>{T(0), T(0), T(0)};
-      const T a0 = rest_value<T>(t.tri_a0, t.tri_a0f, k);
-      const T ar = fdiv(area - a0, a0);
-      T* q = sface + 7 * k;
-      q[0] = third(v0.x + v1.x + v2.x);
-      q[1] = third(v0.y + v1.y + v2.y);
-      q[2] = third(v0.z + v1.z + v2.z);
-      q[3] = (T)t.k_area * (ar + fdiv(ar, fabs(T(kMaxArea) - ar * ar)));
-      q[4] = na.x;
-      q[5] = na.y;
-      q[6] = na.z;
-    }
-    for (int e = tid; e < ne; e += bs) {
-      const int a = t.edges[2 * e], b = t.edges[2 * e + 1];
-      T L;
-      const V3t<T> uv = normalized(ld3(sx, b) - ld3(sx, a), L);
-      const T l0 = rest_value<T>(t.edge_l0, t.edge_l0f, e);
-      const T ef = fdiv(L - l0, l0);
-      V3t<T> fe = vscale(uv, (T)t.k_link * (ef + fdiv(ef, fabs(T(kMaxLink) - ef * ef))));
-      if (visc) {
-        const V3t<T> va = {vv.v[voff + a], vv.v[V + voff + a], vv.v[2 * V + voff + a]};
-        const V3t<T> vb = {vv.v[voff + b], vv.v[V + voff + b], vv.v[2 * V + voff + b]};
-        V3t<T> fv = vscale(vscale(uv, vdot(vb - va, uv)), (T)t.eta_m);
-        const T mm = vnorm(fv);
-        if (mm > T(kForceLimit / 4.0)) fv = vscale(fv, T(kForceLimit / 4.0) / mm);
-        fe = fe + fv;
-      }
-      sedge[3 * e] = fe.x;
-      sedge[3 * e + 1] = fe.y;
-      sedge[3 * e + 2] = fe.z;
-      if (plt) {
-        const V3t<T> pb = plt_bending(sx, t, e);
-        spltb[3 * e] = pb.x;
-        spltb[3 * e + 1] = pb.y;
-        spltb[3 * e + 2] = pb.z;
-      }
-    }
-    if (!plt) {
-      for (int i = tid; i < nv; i += bs) {
-        const int rn = srn[i];
-        const int* rg = t.ring + 6 * i;
-        const V3t<T> xi = ld3(sx, i);
-        V3t<T> sum = {T(0), T(0), T(0)};
-        for (int j = 0; j < rn; ++j) sum = sum + ld3(sx, rg[j]);
-        const V3t<T> dev = V3t<T>{fdiv(sum.x, (T)rn), fdiv(sum.y, (T)rn), fdiv(sum.z, (T)rn)} - xi;
-        V3t<T> pn = {T(0), T(0), T(0)};
-        V3t<T> a = ld3(sx, rg[0]) - xi;
-        const V3t<T> first = a;
-        for (int j = 0; j < rn; ++j) {
-          const V3t<T> b = (j + 1 < rn) ? ld3(sx, rg[j + 1]) - xi : first;
-          T l;
-          pn = pn + normalized(vcross(a, b), l);
-          a = b;
-        }
-        T pl;
-        pn = normalized(pn, pl);
-        const T dDev = fdiv(vdot(pn, dev) - rest_value<T>(t.patch_d0, t.patch_d0f, i), (T)t.edge_mean_eq);
-        const V3t<T> bf = vscale(pn, (T)t.k_bend * (dDev + fdiv(dDev, fabs(T(kMaxBend) - dDev * dDev))));
-        sbf[3 * i] = bf.x;
-        sbf[3 * i + 1] = bf.y;
-        sbf[3 * i + 2] = bf.z;
-      }
-    }
-    block_sum<T>(vol, red);
-    if (tid == 0) {
-      const double volume = red[32] * (1.0 / 6.0);
-      const double vfr = (volume - t.volume_eq) / t.volume_eq;
-      const double vf = -t.k_volume * vfr / fabs(kMaxVol - vfr * vfr);
-      red[31] = vf / t.area_mean_eq;
-    }
-    __syncthreads();
-    const T vforce_per_area = (T)red[31];
-    // --- phase B: gather per vertex
-    for (int i = tid; i < nv; i += bs) {
+  }
+  block_sum<T>(vol, red);  // red[32] = the own faces' sum
+  cluster_sync(cs);
+  const Chunked faces(sface, fch, 4 * sizeof(T)), edges(sedge, ech, sizeof(T)), dihedral(splt, ech, 3 * sizeof(T)),
+      bending(sbf, vch, 3 * sizeof(T));
+  const uint32_t inv_base = smem_addr(sinv);
+  // --- volume constraint in FP64, by one thread of each rank, over the ranks'
+  // sums in their order (the same bits in every rank)
+  if (tid == 0) {
+    const double vfr = (cluster_sum(red + 32, cs) * (1.0 / 6.0) - t.volume_eq) / t.volume_eq;
+    red[33] = -t.k_volume * vfr / fabs(kMaxVol - vfr * vfr) / t.area_mean_eq;
+  }
+  // --- own bending forces, from the unit normals of the incident faces
+  if (!plt) {
+    for (int i = v0 + tid; i < v1; i += bs) {
       const int rn = srn[i];
-      const V3t<T> xi = ld3(sx, i);
-      V3t<T> f = {T(0), T(0), T(0)};
+      V3t<T> sum = {T(0), T(0), T(0)}, pn = {T(0), T(0), T(0)};
 #pragma unroll
       for (int j = 0; j < 6; ++j) {
         if (j >= rn) break;
-        const int r = t.ring[6 * i + j];
-        const T* q = sface + 7 * t.vface[6 * i + j];
-        f = f + vscale(V3t<T>{q[0], q[1], q[2]} - xi, q[3]) + vscale(V3t<T>{q[4], q[5], q[6]}, vforce_per_area);
-        const int e = t.vedge[6 * i + j];
-        const V3t<T> fe = ld3(sedge, e);
-        f = i < r ? f + fe : f - fe;
-        if (!plt) {
-          const T rnr = (T)srn[r];
-          f = f - V3t<T>{fdiv(sbf[3 * r], rnr), fdiv(sbf[3 * r + 1], rnr), fdiv(sbf[3 * r + 2], rnr)};
-        } else {
-          f = f + ld3(spltb, e) - ld3(spltb, t.vopp[6 * i + j]);
-        }
+        sum = sum + ld3(sx, t.ring[6 * i + j]);
+        const int k = t.vface[6 * i + j];
+        const uint32_t owner = faces.owner(k);
+        T q[4], s;
+        ld_cluster4(faces.at(k, owner), q);
+        ld_cluster(cluster_addr(inv_base + (uint32_t)sizeof(T) * faces.within(k, owner), owner), s);
+        pn = pn + vscale(V3t<T>{q[0], q[1], q[2]}, s);
       }
-      if (!plt) f = f + ld3(sbf, i);
-      for (int q = t.vinner_off[i]; q < t.vinner_off[i + 1]; ++q) {
-        const int e = t.vinner[q];
-        const int o = t.inner[2 * e] == i ? t.inner[2 * e + 1] : t.inner[2 * e];
-        const V3t<T> ev = ld3(sx, o) - xi;
-        const T L = vnorm(ev);
-        const V3t<T> uv = {ev.x / L, ev.y / L, ev.z / L};
-        if (t.model == 1) {
-          const T l0 = rest_value<T>(t.inner_l0, t.inner_l0f, e);
-          f = f + vscale(uv, (T)t.k_link * T(5) * ((L - l0) / l0));
-        } else if (t.model == 2) {
-          if (L < T(2) * (T)t.radius) f = f - vscale(vscale(uv, T(1) - L / (T(2) * (T)t.radius)), (T)t.k_cyto);
-          if (L < T(2) * (T)t.core_radius)
-            f = f - vscale(vscale(uv, T(1) - L / (T(2) * (T)t.core_radius)), (T)t.k_inner_rigid);
-        }
-      }
-      vv.f[voff + i] = f.x;
-      vv.f[V + voff + i] = f.y;
-      vv.f[2 * V + voff + i] = f.z;
-      if (M.fuse_spread) spread_vertex(M, voff + i, f);
+      T inv, len;
+      hcnewton::inv_length(vdot(pn, pn), inv, len);
+      const V3t<T> dev = vscale(sum, inv_valence<T>(rn)) - ld3(sx, i);
+      pn = vscale(pn, inv);
+      const T d = quotient(vdot(pn, dev) - rest_value<T>(t.patch_d0, t.patch_d0f, i), (T)t.edge_mean_eq);
+      const T s = (T)t.k_bend * saturating(d, T(kMaxBend));
+      T* q = sbf + 3 * (i - v0);
+      q[0] = pn.x * s;
+      q[1] = pn.y * s;
+      q[2] = pn.z * s;
     }
   }
-  pdl_trigger();
+  cluster_sync(cs);
+  const T push = T(0.5) * (T)red[33];  // volume force per cross product
+  // --- gather the own vertices' forces
+  for (int i = v0 + tid; i < v1; i += bs) {
+    const int rn = srn[i];
+    const V3t<T> xi = ld3(sx, i);
+    V3t<T> f = {T(0), T(0), T(0)}, n = {T(0), T(0), T(0)};
+    T af[6], last = T(0);
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      if (j >= rn) break;
+      const int k = t.vface[6 * i + j];
+      T q[4];
+      ld_cluster4(faces.at(k, faces.owner(k)), q);
+      n = n + V3t<T>{q[0], q[1], q[2]};
+      af[j] = last = q[3];
+    }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      if (j >= rn) break;
+      const int r = t.ring[6 * i + j], e = t.vedge[6 * i + j];
+      T pull;
+      ld_cluster(edges.at(e), pull);
+      // the edge's own scalar and a third of its two faces'
+      const T c = pull + T(1.0 / 3.0) * (af[j] + (j == 0 ? last : af[j - 1]));
+      f = f + vscale(ld3(sx, r) - xi, c);
+      if (!plt) f = f - vscale(ld3_cluster<T>(bending.at(r)), inv_valence<T>(srn[r]));
+      else f = f + ld3_cluster<T>(dihedral.at(e)) - ld3_cluster<T>(dihedral.at(t.vopp[6 * i + j]));
+    }
+    f = f + vscale(n, push);
+    if (!plt) f = f + ld3(sbf, i - v0);
+    for (int q = t.vinner_off[i]; q < t.vinner_off[i + 1]; ++q) {
+      const int e = t.vinner[q];
+      const int o = t.inner[2 * e] == i ? t.inner[2 * e + 1] : t.inner[2 * e];
+      const V3t<T> ev = ld3(sx, o) - xi;
+      T inv, len;
+      hcnewton::inv_length(vdot(ev, ev), inv, len);
+      const V3t<T> uv = vscale(ev, inv);  // toward the partner
+      if (plt) {
+        const T l0 = rest_value<T>(t.inner_l0, t.inner_l0f, e);
+        f = f + vscale(uv, (T)t.k_link * T(5) * quotient(len - l0, l0));
+      } else if (t.model == 2) {
+        const T d1 = T(2) * (T)t.radius, d2 = T(2) * (T)t.core_radius;
+        if (len < d1) f = f - vscale(uv, (T(1) - quotient(len, d1)) * (T)t.k_cyto);
+        if (len < d2) f = f - vscale(uv, (T(1) - quotient(len, d2)) * (T)t.k_inner_rigid);
+      }
+    }
+    vv.f[voff + i] = f.x;
+    vv.f[V + voff + i] = f.y;
+    vv.f[2 * V + voff + i] = f.z;
+    if (M.fuse_spread) spread_vertex(M, voff + i, f);
+  }
+  cluster_sync(cs);  // no rank leaves while another reads its terms
+  end_launch(M);
+}
+
+template <typename T>
+cudaError_t launch_mechanics_staged(const MechView<T>& M, int cluster, int bs, cudaStream_t s) {
+  if (M.ncells <= 0) return cudaSuccess;
+  return launch_cluster(k_mechanics_staged<T>, cluster, dim3(M.ncells * cluster), dim3(bs), M.dyn_smem, s, M.L.pdl,
+                        M.carveout, M);
+}
+size_t mechanics_staged_bytes(int model, int nv, int nf, int ne, int cluster, bool f64) {
+  return f64 ? staged_smem_bytes<double>(model, nv, nf, ne, cluster)
+             : staged_smem_bytes<float>(model, nv, nf, ne, cluster);
 }
 
 // Scatter variant (selected by the tuner): one CTA per cell.  Pass A runs the faces
@@ -1418,32 +1585,62 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 384 : 768) k_mechanics_scatte
   }
 }
 
-// Raise the kernel's dynamic shared-memory limit (done when a cell type is
-// added, never inside a stream capture).
+// Raise the kernels' dynamic shared-memory limits (done when a cell type is
+// added, never inside a stream capture).  The attribute belongs to the kernel,
+// not to a handle: it goes to the device's maximum, so that no handle lowers it
+// beneath what another one launches with.  staged_limit receives the staged
+// kernel's.
 template <typename T>
-cudaError_t prepare_mechanics(int smem_bytes) {
-  cudaError_t e = cudaFuncSetAttribute(k_mechanics<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+cudaError_t prepare_mechanics(int smem_bytes, int* staged_limit) {
+  int dev = 0, optin = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_mechanics_scatter<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+  void (*kernels[3])(const MechView<T>) = {k_mechanics<T>, k_mechanics_scatter<T>, k_mechanics_staged<T>};
+  for (int k = 0; k < 3; ++k) {
+    cudaFuncAttributes a;
+    if ((e = cudaFuncGetAttributes(&a, kernels[k])) != cudaSuccess) return e;
+    const int room = optin - (int)a.sharedSizeBytes;
+    if (k < 2 && smem_bytes > room) return cudaErrorInvalidValue;
+    e = cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize, room);
+    if (e != cudaSuccess) return e;
+    if (k == 2) *staged_limit = room;
+  }
+  e = cudaFuncSetAttribute(k_mechanics<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_mechanics_staged<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+  return cudaFuncSetAttribute(k_mechanics_staged<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
-size_t mechanics_staged_bytes(int model, int nv, int nf, int ne, bool f64) {
-  return f64 ? staged_smem_bytes<double>(model, nv, nf, ne) : staged_smem_bytes<float>(model, nv, nf, ne);
+template <typename T>
+bool mechanics_cluster_fits(bool staged, int cluster, int bs, int smem_bytes) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster);
+  cfg.blockDim = dim3(bs);
+  cfg.dynamicSmemBytes = smem_bytes;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)cluster;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, staged ? k_mechanics_staged<T> : k_mechanics<T>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return n > 0;
 }
 
 // variant 0: vertex-centric gather (deterministic), 1: face/edge scatter with
 // shared-memory atomics
 template <typename T>
-cudaError_t launch_mechanics(const MechView<T>& M, int bs, int grid, int variant, cudaStream_t s) {
+cudaError_t launch_mechanics(const MechView<T>& M, int cluster, int bs, int grid, int variant, cudaStream_t s) {
   if (M.ncells <= 0) return cudaSuccess;
   if (bs <= 0) bs = 256;
   if (bs > (sizeof(T) == 8 ? 384 : 768)) bs = sizeof(T) == 8 ? 384 : 768;
   if (grid <= 0 || grid > M.ncells) grid = M.ncells;
   if (variant == 1) return launch_kernel(k_mechanics_scatter<T>, dim3(grid), dim3(bs), M.dyn_smem, s, M.L.pdl, M);
-  if (variant == 2) return launch_kernel(k_mechanics_staged<T>, dim3(grid), dim3(bs), M.dyn_smem, s, M.L.pdl, M);
-  return launch_kernel(k_mechanics<T>, dim3(grid), dim3(bs), M.dyn_smem, s, M.L.pdl, M);
+  return launch_cluster(k_mechanics<T>, cluster, dim3(grid * cluster), dim3(bs), M.dyn_smem, s, M.L.pdl, M.carveout, M);
 }
 
 // device [3][Vcap] (T) -> [V][3] double
@@ -1762,9 +1959,11 @@ cudaError_t launch_tile_sort(const int* offsets, int* tile_vertices, const int* 
                                                    cudaStream_t);                                              \
   template cudaError_t launch_interp_advance<T>(const LbmView<T>&, const VertexView<T>&, const TileGrid&, int, \
                                                 int, int, cudaStream_t);                                       \
-  template cudaError_t launch_mechanics<T>(const MechView<T>&, int, int, int, cudaStream_t);                   \
-  template size_t mechanics_smem_bytes<T>(int);                                                                \
-  template cudaError_t prepare_mechanics<T>(int);                                                              \
+  template cudaError_t launch_mechanics<T>(const MechView<T>&, int, int, int, int, cudaStream_t);              \
+  template cudaError_t launch_mechanics_staged<T>(const MechView<T>&, int, int, cudaStream_t);                \
+  template size_t mechanics_smem_bytes<T>(int, int);                                                           \
+  template cudaError_t prepare_mechanics<T>(int, int*);                                                        \
+  template bool mechanics_cluster_fits<T>(bool, int, int, int);                                                \
   template cudaError_t launch_soa_to_aos<T>(const T*, double*, long long, int, cudaStream_t);                  \
   template cudaError_t launch_bin_vertices<T>(const LbmView<T>&, const VertexView<T>&, const TileGrid&,         \
                                               cudaStream_t);

@@ -135,6 +135,8 @@ struct TypeDev {
   const float* slot_l0f;
   const double* tri_a0;
   const double* edge_l0;
+  const double* tri_ia0;  // reciprocals of tri_a0 and edge_l0 (FP64 handles only)
+  const double* edge_il0;
   const double* edge_angle0;
   const double* patch_d0;
   const double* inner_l0;
@@ -205,6 +207,12 @@ struct MechView {
   // interpolates and advances its cell's vertices first (with fuse_spread,
   // which then tags with stamp + 1)
   int fuse_advance;
+  // the launches of several cell types side by side: after_prev, this one was
+  // launched programmatically behind the previous type's, whose results it does
+  // not read: it does not wait for them at its start but does not end before
+  // them; before_next, it lets the next type's start as soon as its own CTAs run
+  int after_prev, before_next;
+  int carveout;  // shared memory of the SMs it runs on, in percent (0: what the launch takes)
   TileGrid tg;
   LbmView<T> L;
   T f_limit;
@@ -212,21 +220,39 @@ struct MechView {
 
 
 // Kernel launch with or without programmatic dependent launch (the kernel
-// then starts with pdl_wait, see hc_async.cuh).
+// then starts with pdl_wait, see hc_async.cuh), in clusters of CTAs along x.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_kernel(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl,
-                          Args... args) {
+cudaError_t launch_cluster(void (*k)(KArgs...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                           bool pdl, int carveout, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchAttribute attr[3];
+  int n = 0;
+  if (pdl) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = (unsigned)cluster;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    n++;
+  }
+  if (carveout > 0) {
+    attr[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[n++].val.sharedMemCarveout = (unsigned)carveout;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, k, args...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_kernel(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl,
+                          Args... args) {
+  return launch_cluster(k, 1, grid, block, smem, s, pdl, 0, args...);
 }
 
 // Launch wrappers; each enqueues on `s` and returns the launch error code.
@@ -287,14 +313,22 @@ cudaError_t launch_add_vertex_forces(const VertexView<T>& vv, const int* ids, co
 template <typename T>
 cudaError_t launch_interp_advance(const LbmView<T>& L, const VertexView<T>& vv, const TileGrid& tg,
                                   int do_interp, int do_advance, int bs, cudaStream_t s);
-// shared memory the staged force assembly (variant 2) needs for one cell type
-size_t mechanics_staged_bytes(int model, int nv, int nf, int ne, bool f64);
+// shared memory a CTA of the staged force assembly (variant 2) needs for one
+// cell type split over `cluster` CTAs
+size_t mechanics_staged_bytes(int model, int nv, int nf, int ne, int cluster, bool f64);
 template <typename T>
-cudaError_t launch_mechanics(const MechView<T>& M, int bs, int grid, int variant, cudaStream_t s);
+cudaError_t launch_mechanics(const MechView<T>& M, int cluster, int bs, int grid, int variant, cudaStream_t s);
+// variant 2: each cell on a cluster of 1, 2, 4, 8 or 16 CTAs of bs threads (at
+// most 384)
 template <typename T>
-size_t mechanics_smem_bytes(int nv);
+cudaError_t launch_mechanics_staged(const MechView<T>& M, int cluster, int bs, cudaStream_t s);
+// whether the device can hold a cluster of the staged or vertex-centric kernel
 template <typename T>
-cudaError_t prepare_mechanics(int smem_bytes);
+bool mechanics_cluster_fits(bool staged, int cluster, int bs, int smem_bytes);
+template <typename T>
+size_t mechanics_smem_bytes(int nv, int cluster);
+template <typename T>
+cudaError_t prepare_mechanics(int smem_bytes, int* staged_limit);
 template <typename T>
 cudaError_t launch_soa_to_aos(const T* src, double* dst, long long V, int n, cudaStream_t s);
 template <typename T>

@@ -44,6 +44,17 @@ HC_POS_HD void double_words(double x, uint32_t& hi, uint32_t& lo) {
 #endif
 }
 
+HC_POS_HD double double_from_words(uint32_t hi, uint32_t lo) {
+#ifdef __CUDA_ARCH__
+  return __hiloint2double((int)hi, (int)lo);
+#else
+  const uint64_t b = ((uint64_t)hi << 32) | lo;
+  double x;
+  memcpy(&x, &b, sizeof x);
+  return x;
+#endif
+}
+
 HC_POS_HD float float_from_bits(uint32_t b) {
 #ifdef __CUDA_ARCH__
   return __uint_as_float(b);
@@ -102,6 +113,20 @@ HC_POS_HD bool fraction_bits(double P, FractionBits& b) {
   b.fh = mh & ((1u << t) - 1u);
   b.fl = lo;
   b.up = (int)((b.fh >> (t - 1)) & 1u);
+  return true;
+}
+
+// For 1 <= P < 2^20: floor(P) as an integer and as a double (the significand
+// with its fraction bits cleared; they reach into the high word).  Returns
+// false for every other P.
+HC_POS_HD bool floor_bits(double P, int& q, double& q0) {
+  uint32_t hi, lo;
+  double_words(P, hi, lo);
+  const int be = (int)(hi >> 20);
+  if ((unsigned)(be - 1023) > 19u) return false;
+  const int t = 1043 - be;  // fraction bits in the high word, 1..20
+  q = (int)(((hi & 0xFFFFFu) | 0x100000u) >> t);
+  q0 = double_from_words(hi & ~((1u << t) - 1u), 0u);
   return true;
 }
 

@@ -276,12 +276,16 @@ int hc_device_status(hc_handle* h, unsigned int* status);
 /* --- launch tuning (project autotuner; results cached on disk) */
 int hc_autotune(hc_handle* h, const char* cache_path);
 int hc_get_tuning(hc_handle* h, int* out8);
-/* in8: collide-stream block (bx, by; bx = 0 whole rows, else 8 or 16, whose
+/* until hc_set_tuning or hc_autotune, the launch shapes follow the lattice and
+ * its cells; hc_get_tuning returns the ones in use.
+ * in8: collide-stream block (bx, by; bx = 0 whole rows, else 8 or 16, whose
  * warps are 8 x 4 or 16 x 2 tiles, or a multiple of 32; whole warps, at most
  * 256 threads), spread block,
- * interpolation block, mechanics block, mechanics grid (0 = one CTA per cell),
- * mechanics variant (0 vertex gather, 1 face/edge scatter, 2 staged face/edge
- * terms gathered per vertex), and in8[7]: bits 0-7 the collide-stream kind
+ * interpolation block, mechanics block (variant 2: of cells that one CTA
+ * assembles, at most 384), mechanics grid (0 = one CTA per cell, or one cluster
+ * of CTAs where the cells are few or large; variant 2 always), mechanics variant
+ * (0 vertex gather, 1 face/edge scatter, 2 staged face/edge terms gathered per
+ * vertex), and in8[7]: bits 0-7 the collide-stream kind
  * (0 (x,y)-blocks or rows, 1 one thread per fluid node, else bulk copies:
  * stages | CTAs per SM << 4), bits 8-9 the node velocity (0 every tagged node,
  * 1 per fluid node, 2 over warp-packed tagged nodes, 3 every fluid node in
