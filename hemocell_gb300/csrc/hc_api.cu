@@ -107,7 +107,7 @@ struct hc_handle {
   // lattice units, timescales (0 = off) and device state
   double rep_k = 0, rep_rc = 0, brep_k = 0, brep_rc = 0;
   int rep_every = 0, brep_every = 0;
-  int* rep_cnt = nullptr;
+  int2* rep_cnt = nullptr;
   int* rep_slot = nullptr;
   int* rep_vq = nullptr;
   void* rep_xr = nullptr;
@@ -604,13 +604,13 @@ int ensure_repulsion(hc_handle* h) {
   const bool any = h->rep_every > 0 || h->brep_every > 0;
   if (!any) return HC_OK;
   if (h->rep_every > 0 && !h->rep_cnt) {
-    HC_CUDA(h, dalloc(h, (void**)&h->rep_cnt, sizeof(int) * h->N));
+    HC_CUDA(h, dalloc(h, (void**)&h->rep_cnt, sizeof(int2) * h->N));
     HC_CUDA(h, dalloc(h, (void**)&h->rep_slot, sizeof(int) * hcd::REP_SLOTS * h->N));
   }
   const long long cap = std::max<long long>(h->Vcap, 1);
   if (h->rep_vcap < cap || !h->rep_vq) {
     if ((rc = grow1(h, (void**)&h->rep_vq, 4, h->rep_vcap, cap, 0)) != HC_OK) return rc;
-    if ((rc = grow3(h, &h->rep_xr, h->ts, h->rep_vcap, cap, 0)) != HC_OK) return rc;
+    if ((rc = grow1(h, &h->rep_xr, 4 * h->ts, h->rep_vcap, cap, 0)) != HC_OK) return rc;
     const int kept = (int)std::min<long long>(h->nvert, h->rep_vcap);
     if ((rc = grow3(h, &h->frep_cell, h->ts, h->rep_vcap, cap, h->frep_cell ? kept : 0)) != HC_OK) return rc;
     if ((rc = grow3(h, &h->frep_wall, h->ts, h->rep_vcap, cap, h->frep_wall ? kept : 0)) != HC_OK) return rc;
@@ -753,12 +753,12 @@ int enq_repulsion(hc_handle* h, int it, bool force = false) {
   const bool dc = h->rep_every > 0 && (force || it % h->rep_every == 0);
   const bool dw = h->brep_every > 0 && (force || it % h->brep_every == 0);
   if ((!dc && !dw) || h->nvert == 0) return HC_OK;
-  if (dc) HC_CUDA(h, cudaMemsetAsync(h->rep_cnt, 0, sizeof(int) * h->N, h->stream));
+  if (dc) HC_CUDA(h, cudaMemsetAsync(h->rep_cnt, 0, sizeof(int2) * h->N, h->stream));
   hcd::RepView<T> R;
-  R.cnt = dc ? h->rep_cnt : nullptr;
+  R.node = dc ? h->rep_cnt : nullptr;
   R.slot = h->rep_slot;
   R.vq = h->rep_vq;
-  R.xr = (T*)h->rep_xr;
+  R.rec = (hcd::RepRecord<T>*)h->rep_xr;
   R.bnode = h->rep_bnode;
   R.fcell = dc ? (T*)h->frep_cell : nullptr;
   R.fwall = dw ? (T*)h->frep_wall : nullptr;
@@ -2071,6 +2071,24 @@ int hc_set_boundary_repulsion(hc_handle* h, double k, double cutoff, int every) 
               if (!out && h->hflag[q[0] + (long long)h->nx * (q[1] + (long long)h->ny * q[2])] == 0) near_fluid = true;
             }
         b[n] = near_fluid ? 1 : 0;
+      }
+  // bit 1: the node or one of its 26 neighbours is a boundary node
+  for (int Z = 0; Z < h->nz; ++Z)
+    for (int Y = 0; Y < h->ny; ++Y)
+      for (int X = 0; X < h->nx; ++X) {
+        if (!(b[X + (long long)h->nx * (Y + (long long)h->ny * Z)] & 1)) continue;
+        for (int dz = -1; dz <= 1; ++dz)
+          for (int dy = -1; dy <= 1; ++dy)
+            for (int dx = -1; dx <= 1; ++dx) {
+              int q[3] = {X + dx, Y + dy, Z + dz};
+              bool out = false;
+              for (int a = 0; a < 3; ++a)
+                if (q[a] < 0 || q[a] >= dims[a]) {
+                  if (h->p.periodic[a]) q[a] = (q[a] + dims[a]) % dims[a];
+                  else out = true;
+                }
+              if (!out) b[q[0] + (long long)h->nx * (q[1] + (long long)h->ny * q[2])] |= 2;
+            }
       }
   if (!h->rep_bnode) HC_CUDA(h, dalloc(h, (void**)&h->rep_bnode, h->N));
   HC_CUDA(h, cudaMemcpyAsync(h->rep_bnode, b.data(), h->N, cudaMemcpyHostToDevice, h->stream));

@@ -174,12 +174,19 @@ constexpr int REP_SLOTS = 10;
 constexpr unsigned int STATUS_REP_OVERFLOW = 8u;
 
 template <typename T>
+struct alignas(4 * sizeof(T)) RepRecord {
+  T x, y, z;
+  int cell;
+};
+
+template <typename T>
 struct RepView {
-  int* cnt;              // [N] vertices binned per node (null: no inter-cell term)
+  int2* node;            // [N] vertices binned per node; their cell plus one, 0 none, -1 several
+                         // (null: no inter-cell term)
   int* slot;             // [N][REP_SLOTS]
   int* vq;               // [V] node of each vertex, -1 when not binned
-  T* xr;                 // [3][V] position relative to that node
-  const uint8_t* bnode;  // [N] 1 on boundary nodes (wall term)
+  RepRecord<T>* rec;     // [V] position relative to that node, and the cell
+  const uint8_t* bnode;  // [N] bit 0 on boundary nodes (wall term), bit 1 where one of the 27 is
   T* fcell;              // [3][V] inter-cell term to recompute (null: keep)
   T* fwall;              // [3][V] wall term to recompute (null: keep)
   T kc, rc, kw, rw;      // constants and cutoffs (lattice units)
