@@ -324,6 +324,7 @@ LbmView<T> lbm_view(hc_handle* h, int src, int fcur) {
   L.stamp = h->stamp;
   L.reverse = src;  // alternates with the buffer parity
   L.ck = hcd::collide_constants<T>((T)(1.0 / h->u.tau));
+  L.relax = hcfix::relax_constants(1.0 / h->u.tau);
   for (int c = 0; c < hcd::MAX_WALL_CLASSES; ++c)
     for (int a = 0; a < 3; ++a) L.uw[c][a] = (T)h->uw[c][a];
   L.status = h->status;
@@ -365,8 +366,8 @@ VertexView<T> vertex_view(hc_handle* h) {
 // hc_autotune), from its lattice and cells.  Steps in microseconds, this choice
 // against the other side of the line:
 //   Collide-stream in FP64: over the fluid-node list, as a warp with one fluid
-//   node costs the FP64 pipe as much as a full one (pipe 64x64x256 206 against
-//   273 for the kernel, 150^3 Couette box 904 against 967).
+//   node costs the issue slots as much as a full one (pipe 64x64x256 82 against
+//   110 for the kernel, 150^3 Couette box 338 against 384).
 //   In FP32: (x, y)-blocks, or the list where rows rounded up to warps idle a
 //   twentieth of their lanes (rows of 64: 92 against 96; of 97: 29 against 32; of
 //   181: 65 against 67); evict-last population stores (pipe 92 against 96,
@@ -375,7 +376,7 @@ VertexView<T> vertex_view(hc_handle* h) {
 //   with 80 RBCs 78 against 81; with 20 65 against 72 the other way), else the
 //   tagged nodes packed into warps from half a million nodes on (128^3 with 6
 //   RBCs 96 against 101; 64^3 with 8 36.9 against 35.8).  In FP64 tagged fluid
-//   nodes (pipe 453; every node 482, packed 449; 50^3 box 94, 109, 96).
+//   nodes (pipe 294; every node 297, packed 297; 50^3 box 58, 66, 60).
 //   Programmatic launch always (32^3 box 28.7 against 30.5; FP64 50^3 box 82
 //   against 94).
 //   Force assembly: variant 2 (see mech_plan).

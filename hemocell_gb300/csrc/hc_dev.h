@@ -12,6 +12,8 @@
 
 #include <string>
 
+#include "hc_blockfixed.h"
+
 namespace hcd {
 
 constexpr uint32_t NB_SOLID = 1u << 23;     // node itself is a wall node
@@ -57,6 +59,7 @@ struct LbmView {
   uint32_t* stamp;               // device step stamp (advanced by interp_advance)
   int reverse;                   // sweep the lattice from the last z-plane down
   CollideK<T> ck;
+  hcfix::Relax relax;  // the block fixed-point collision's (FP64 form)
   T uw[MAX_WALL_CLASSES][3];
   // 32-bit pull offsets, valid when 19 N < 2^31 (fast != 0): population j of
   // an interior node n (no wrap, no bounce-back link) is fsrc[n + off[j]]

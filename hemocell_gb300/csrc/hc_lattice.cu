@@ -14,29 +14,24 @@
 
 namespace hcd {
 
-// Guo-forced BGK collision of one node from its pulled populations f and
-// force F; writes the post-collision populations and the node's next force
-// (the body force of plane Z).
-template <typename T, typename Idx, bool KEEP = false>
-__device__ __forceinline__ void collide_store(const LbmView<T>& L, Idx n, int Z, const T f[19], T Fx, T Fy, T Fz) {
+// The collision in T arithmetic: the FP32 form's, and the FP64 form's at nodes
+// that the block fixed-point collision refuses.
+template <typename T, typename Idx, bool KEEP>
+__device__ __forceinline__ void collide_float(const LbmView<T>& L, Idx n, const T f[19], T Fx, T Fy, T Fz) {
   const Idx N = (Idx)L.N;
-  if (!HC_IN(L.status, n, N) || !HC_IN(L.status, Z, L.nz)) return;
   uint64_t pol = 0;
   if constexpr (KEEP) pol = l2_policy_evict_last();
   T rhoBar, jx, jy, jz;
   moments(f, rhoBar, jx, jy, jz);
   if constexpr (sizeof(T) == 8) {
-    // FP64: the FP64 pipe bounds this kernel, so the fewest operations.  With
+    // FP64: the FP64 pipe would bound this, so the fewest operations.  With
     // m = rho u = j + F/2 and opposite velocities c, -c of weight w, the
     // equilibrium and Guo source of the pair are P + Q and P - Q:
     //   P = w [om (rhoBar - 1.5 m.u) - 3 hs u.F] + (c.u) (c.a)
     //   Q = c.b,   a = w (4.5 om m + 9 hs F),   b = w (3 om m + 3 hs F)
     // (hs = 1 - om/2).  Both quadratic terms of P share the factor c.u, so a
     // diagonal pair costs three sums and one multiply-add for P and Q instead
-    // of two sums, two products and three multiply-adds: 146 FP64 instructions
-    // a node where the expression by equilibrium and source took 206.  The
-    // 64x64x256 pipe's (x, y)-block kernel goes from 371 to 273 us, the 150^3
-    // Couette box's (moving walls) from 1620 to 967 us.  FP32 keeps the longer
+    // of two sums, two products and three multiply-adds.  FP32 keeps the longer
     // form below: its rounding is the smaller one of the two (velocity error of
     // 600 steps 4.7e-6 against 7.5e-6), and arithmetic does not bound it.
     const T invRho = T(1) / (T(1) + rhoBar);
@@ -99,6 +94,36 @@ __device__ __forceinline__ void collide_store(const LbmView<T>& L, Idx n, int Z,
       st_pop<KEEP>(L.fdst + i * N + n, om1 * f[i] + (P - Q), pol);
     }
   }
+}
+template <typename Idx, bool KEEP>
+__device__ __noinline__ void collide_refused(const LbmView<double>& L, Idx n, int X, int Y, int Z, uint32_t m) {
+  double f[19], Fx, Fy, Fz;
+  pull(L, L.fsrc, X, Y, Z, (long long)n, m, f);
+  FieldLayout<double>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
+  collide_float<double, Idx, KEEP>(L, n, f, Fx, Fy, Fz);
+}
+
+// Guo-forced BGK collision of node (X, Y, Z) with mask m from its pulled
+// populations f and force F; writes the post-collision populations and the node's
+// next force (the body force of plane Z).
+// FP64 runs in block fixed point (hc_blockfixed.h): the FP64 pipe bounded the
+// kernel at 143 instructions a node (206 before the pair terms shared c.u).  The
+// pipe 64x64x256: 371 us by equilibrium and source, 206 in FP64 over the fluid
+// list, 83 now; the 150^3 Couette box 1620, 904 and 338 us.
+template <typename T, typename Idx, bool KEEP = false>
+__device__ __forceinline__ void collide_store(const LbmView<T>& L, Idx n, int X, int Y, int Z, uint32_t m,
+                                              const T f[19], T Fx, T Fy, T Fz) {
+  const Idx N = (Idx)L.N;
+  if (!HC_IN(L.status, n, N) || !HC_IN(L.status, Z, L.nz)) return;
+  if constexpr (sizeof(T) == 8) {
+    uint64_t pol = 0;
+    if constexpr (KEEP) pol = l2_policy_evict_last();
+    T* const dst = L.fdst + n;
+    if (!hcfix::collide(f, Fx, Fy, Fz, L.relax, [&](int i, double v) { st_pop<KEEP>(dst + i * N, v, pol); }))
+      collide_refused<Idx, KEEP>(L, n, X, Y, Z, m);
+  } else {
+    collide_float<T, Idx, KEEP>(L, n, f, Fx, Fy, Fz);
+  }
   FieldLayout<T>::store(L.Fnext, N, n, L.bodyz[Z], L.bodyz[L.nz + Z], L.bodyz[2 * L.nz + Z]);
 }
 
@@ -156,7 +181,7 @@ __global__ void __launch_bounds__(256, kCollideBlocks<T>) k_collide_stream(const
   }
   T Fx, Fy, Fz;
   FieldLayout<T>::load(L.Fcur, N, n, Fx, Fy, Fz);
-  collide_store<T, Idx, (V & 2) != 0>(L, n, Z, f, Fx, Fy, Fz);
+  collide_store<T, Idx, (V & 2) != 0>(L, n, X, Y, Z, m, f, Fx, Fy, Fz);
   pdl_trigger();
 }
 
@@ -190,7 +215,7 @@ __global__ void __launch_bounds__(256, kCollideBlocks<T>) k_collide_stream_fluid
   else pull(L, L.fsrc, X, Y, Z, (long long)n, m, f);
   T Fx, Fy, Fz;
   FieldLayout<T>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
-  collide_store<T, int, (V & 2) != 0>(L, n, Z, f, Fx, Fy, Fz);
+  collide_store<T, int, (V & 2) != 0>(L, n, X, Y, Z, m, f, Fx, Fy, Fz);
   pdl_trigger();
 }
 
@@ -334,7 +359,7 @@ __global__ void __launch_bounds__(256) k_collide_stream_bulk(const LbmView<T> L,
         Fy = fp[RN + tid];
         Fz = fp[2 * RN + tid];
       }
-      collide_store<T, long long>(L, n, Z, f, Fx, Fy, Fz);
+      collide_store<T, long long>(L, n, X, Y, Z, m, f, Fx, Fy, Fz);
     }
     if (__syncthreads_or(!ok)) {
       failed = true;
@@ -445,24 +470,36 @@ cudaError_t launch_collide_stream(const LbmView<T>& L, int bx, int by, cudaStrea
 // tagged by this step's stencils (Palabos computeVelocity for Guo forcing,
 // core/hemoCellParticleField.cpp:833); L.fsrc is the post-collision state,
 // L.Fcur the force of that collision.
-// FP64 takes one reciprocal of rho for the three components, as the collision
-// does: an FP64 division is about ten instructions of the pipe that bounds the
-// kernel.
+// The FP64 form sums in block fixed point, as its collision does; a node that
+// refuses (values that are not finite, rho far from one) takes FP64.
+__device__ __noinline__ void velocity_refused(const LbmView<double>& L, long long n, int X, int Y, int Z, uint32_t m) {
+  double f[19], rhoBar, jx, jy, jz, Fx, Fy, Fz;
+  pull(L, L.fsrc, X, Y, Z, n, m, f);
+  moments(f, rhoBar, jx, jy, jz);
+  FieldLayout<double>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
+  const double inv = 1.0 / (1.0 + rhoBar);
+  FieldLayout<double>::store(L.unode, L.N, n, (jx + 0.5 * Fx) * inv, (jy + 0.5 * Fy) * inv, (jz + 0.5 * Fz) * inv);
+}
 template <typename T>
-__device__ __forceinline__ void store_velocity(const LbmView<T>& L, long long n, T rhoBar, T jx, T jy, T jz, T Fx, T Fy,
-                                               T Fz) {
-  const T rho = T(1) + rhoBar;
-  const T mx = jx + T(0.5) * Fx, my = jy + T(0.5) * Fy, mz = jz + T(0.5) * Fz;
+__device__ __forceinline__ void store_velocity(const LbmView<T>& L, long long n, int X, int Y, int Z, uint32_t m,
+                                               const T f[19]) {
+  T Fx, Fy, Fz;
+  FieldLayout<T>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
   if constexpr (sizeof(T) == 8) {
-    const T inv = T(1) / rho;
-    FieldLayout<T>::store(L.unode, L.N, n, mx * inv, my * inv, mz * inv);
+    T ux, uy, uz;
+    if (hcfix::velocity(f, Fx, Fy, Fz, ux, uy, uz)) FieldLayout<T>::store(L.unode, L.N, n, ux, uy, uz);
+    else velocity_refused(L, n, X, Y, Z, m);
   } else {
-    FieldLayout<T>::store(L.unode, L.N, n, mx / rho, my / rho, mz / rho);
+    T rhoBar, jx, jy, jz;
+    moments(f, rhoBar, jx, jy, jz);
+    const T rho = T(1) + rhoBar;
+    FieldLayout<T>::store(L.unode, L.N, n, (jx + T(0.5) * Fx) / rho, (jy + T(0.5) * Fy) / rho,
+                          (jz + T(0.5) * Fz) / rho);
   }
 }
 
 template <typename T, bool I32>
-__global__ void __launch_bounds__(256) k_node_velocity(const LbmView<T> L) {
+__global__ void __launch_bounds__(256, 4) k_node_velocity(const LbmView<T> L) {
   pdl_wait();
   using Idx = typename std::conditional<I32, int, long long>::type;
   const Idx g = (Idx)blockIdx.x * blockDim.x + threadIdx.x;
@@ -475,14 +512,11 @@ __global__ void __launch_bounds__(256) k_node_velocity(const LbmView<T> L) {
   T f[19];
   if (I32 && pull_is_inline(L, X, Y, Z, m)) pull_inline(L, L.fsrc, (int)n, X, Y, Z, m, f);
   else pull(L, L.fsrc, X, Y, Z, (long long)n, m, f);
-  T rhoBar, jx, jy, jz, Fx, Fy, Fz;
-  moments(f, rhoBar, jx, jy, jz);
-  FieldLayout<T>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
-  store_velocity(L, n, rhoBar, jx, jy, jz, Fx, Fy, Fz);
+  store_velocity(L, n, X, Y, Z, m, f);
   pdl_trigger();
 }
 template <typename T>
-__global__ void __launch_bounds__(256) k_node_velocity_fluid(const LbmView<T> L) {
+__global__ void __launch_bounds__(256, 4) k_node_velocity_fluid(const LbmView<T> L) {
   pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= L.nfluid) return;
@@ -494,10 +528,7 @@ __global__ void __launch_bounds__(256) k_node_velocity_fluid(const LbmView<T> L)
   T f[19];
   if (pull_is_inline(L, X, Y, Z, m)) pull_inline(L, L.fsrc, n, X, Y, Z, m, f);
   else pull(L, L.fsrc, X, Y, Z, (long long)n, m, f);
-  T rhoBar, jx, jy, jz, Fx, Fy, Fz;
-  moments(f, rhoBar, jx, jy, jz);
-  FieldLayout<T>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
-  store_velocity(L, n, rhoBar, jx, jy, jz, Fx, Fy, Fz);
+  store_velocity(L, n, X, Y, Z, m, f);
   pdl_trigger();
 }
 
@@ -514,14 +545,11 @@ __device__ __forceinline__ void node_velocity_at(const LbmView<T>& L, int n) {
   T f[19];
   if (pull_is_inline(L, X, Y, Z, m)) pull_inline(L, L.fsrc, n, X, Y, Z, m, f);
   else pull(L, L.fsrc, X, Y, Z, (long long)n, m, f);
-  T rhoBar, jx, jy, jz, Fx, Fy, Fz;
-  moments(f, rhoBar, jx, jy, jz);
-  FieldLayout<T>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
-  store_velocity(L, n, rhoBar, jx, jy, jz, Fx, Fy, Fz);
+  store_velocity(L, n, X, Y, Z, m, f);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_node_velocity_packed(const LbmView<T> L) {
+__global__ void __launch_bounds__(256, 4) k_node_velocity_packed(const LbmView<T> L) {
   pdl_wait();
   __shared__ int list[8][256];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -567,7 +595,7 @@ __global__ void __launch_bounds__(256) k_node_velocity_packed(const LbmView<T> L
 // holds both kinds of node (every warp of a lattice with walls across its
 // rows) then issues one sequence of 19 loads instead of both.
 template <typename T, bool MW, bool INTERIOR>
-__global__ void __launch_bounds__(256) k_node_velocity_dense(const LbmView<T> L) {
+__global__ void __launch_bounds__(256, 4) k_node_velocity_dense(const LbmView<T> L) {
   pdl_wait();
   const int X = blockIdx.x * blockDim.x + threadIdx.x;
   const int Y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -580,10 +608,7 @@ __global__ void __launch_bounds__(256) k_node_velocity_dense(const LbmView<T> L)
   if (INTERIOR && (m & NB_INTERIOR)) pull_interior(L, L.fsrc, n, f);
   else if (pull_is_inline(L, X, Y, Z, m)) pull_inline<T, MW>(L, L.fsrc, n, X, Y, Z, m, f);
   else pull(L, L.fsrc, X, Y, Z, (long long)n, m, f);
-  T rhoBar, jx, jy, jz, Fx, Fy, Fz;
-  moments(f, rhoBar, jx, jy, jz);
-  FieldLayout<T>::load(L.Fcur, L.N, n, Fx, Fy, Fz);
-  store_velocity(L, n, rhoBar, jx, jy, jz, Fx, Fy, Fz);
+  store_velocity(L, n, X, Y, Z, m, f);
   pdl_trigger();
 }
 
