@@ -57,6 +57,7 @@ struct hc_handle {
   int cur = 0;
   uint32_t* nbmask = nullptr;
   uint8_t* flag = nullptr;
+  uint8_t* corner = nullptr;
   uint32_t* ntag = nullptr;
   void* unode = nullptr;
   uint32_t* stamp = nullptr;
@@ -318,6 +319,7 @@ LbmView<T> lbm_view(hc_handle* h, int src, int fcur) {
   L.Fnext = (T*)h->F[1 - fcur];
   L.nbmask = h->nbmask;
   L.flag = h->flag;
+  L.corner = h->corner;
   L.bodyz = (const T*)h->bodyz;
   L.ntag = tags_needed(h, h->tune) ? h->ntag : nullptr;
   L.unode = (T*)h->unode;
@@ -455,6 +457,7 @@ int upload_flags(hc_handle* h) {
   std::vector<uint32_t> mask;
   build_nbmask(h, mask);
   HC_CUDA(h, cudaMemcpyAsync(h->flag, h->hflag.data(), h->N, cudaMemcpyHostToDevice, h->stream));
+  HC_CUDA(h, hcd::launch_corner_flags(h->flag, h->corner, h->nx, h->ny, h->nz, h->stream));
   HC_CUDA(h, cudaMemcpyAsync(h->nbmask, mask.data(), 4 * h->N, cudaMemcpyHostToDevice, h->stream));
   // the fluid-node list, when coordinates pack into 10/10/12 bits and every
   // population index fits 32 bits
@@ -792,13 +795,13 @@ size_t gather_bytes(const hc_handle* h, const TypeSlot& ts, int cluster = 1) {
 // least, 4 up to three CTAs an SM (two where other types' CTAs need room beside
 // them: 110 RBCs with 11 platelets and a WBC take 162 us a step on 4 CTAs a
 // cell, some of which then wait for a second wave), 8 up to two.  Either form takes 16 where 8
-// would leave a CTA more than 96 vertices.  Measured in microseconds a step,
-// staged, with the advance and spread in it, n RBCs of 642 vertices on
-// 1 / 2 / 4 / 8 CTAs a cell:
-//   FP64  n = 30: 112 / 61 / 51 / 49    110: 112 / 98 / 90 / 133
-//         n = 220: 199 / 147 / 165 / 220    280: 198 / 187 / 231 / 256
-//   FP32  n = 30: 34 / 30 / 29 / 31     60: 34 / 30 / 36 / 41
-//         n = 110: 35 / 40 / 48 / 54    280: 48 / 79 / 112 / 141
+// would leave a CTA more than 96 vertices.  The kernel in microseconds, staged,
+// with the advance and spread in it, n RBCs of 642 vertices on 1 / 2 / 4 / 8 CTAs
+// a cell:
+//   FP64  n = 30: 103 / 60 / 49 / 48    110: 105 / 96 / 87 / 128
+//         n = 220: 182 / 143 / 161 / 214    280: 182 / 181 / 223 / 249
+//   FP32  n = 30: 27 / 26 / 26 / 27     60: 27 / 27 / 31 / 36
+//         n = 110: 28 / 35 / 41 / 65    280: 39 / 68 / 108 / 130
 // Threads, staged: one per face of the CTA's share, 128 to 384 (256 from four
 // CTAs a cell on); the 384 of a whole RBC are two CTAs an SM.
 // An FP32 type whose terms, face by face and edge by edge, took more than 110 KB
@@ -832,7 +835,7 @@ MechPlan mech_plan(const hc_handle* h, const TypeSlot& ts) {
   if (cs == 8 && nv > 8 * 96 && 16 * n <= h->sms && ts.cluster16) cs = 16;
   const size_t whole = 4 * (6 * (size_t)nv + 7 * (size_t)nf + 3 * (size_t)ne * (model == HC_MODEL_PLT_SIMPLE ? 2 : 1)) +
                        (size_t)nv + 272;
-  if (h->tune[6] == 2 && (h->f64 || (whole <= 110 * 1024 && (h->tuned || !few_small(h))))) {
+  if (h->tune[6] == 2 && nf < 65536 && ne < 65536 && (h->f64 || (whole <= 110 * 1024 && (h->tuned || !few_small(h))))) {
     int c = cs;
     while (c < 8 && bytes(c) > (size_t)h->staged_limit) c *= 2;
     if (bytes(c) <= (size_t)h->staged_limit) {
@@ -1651,6 +1654,7 @@ hc_handle* hc_create(const hc_params* p) {
     cudaMemcpyAsync(h->stamp, &one, 4, cudaMemcpyHostToDevice, h->stream);
   }
   if (dalloc(h, (void**)&h->nbmask, 4 * h->N) != cudaSuccess || dalloc(h, (void**)&h->flag, h->N) != cudaSuccess ||
+      dalloc(h, (void**)&h->corner, h->N) != cudaSuccess ||
       dalloc(h, &h->bodyz, 3 * h->ts * h->nz) != cudaSuccess ||
       dalloc(h, (void**)&h->dtypes, sizeof(TypeDev) * hcd::MAX_TYPES) != cudaSuccess ||
       dalloc(h, (void**)&h->status, sizeof(unsigned int)) != cudaSuccess)
@@ -1676,7 +1680,7 @@ int hc_destroy(hc_handle* h) {
     dfree(h, ts.blob);
     dfree(h, ts.dcells);
   }
-  void* ptrs[] = {h->ntag, h->unode, h->stamp, h->nbmask, h->flag,  h->bodyz,     h->dtypes,     h->x,          h->v,
+  void* ptrs[] = {h->ntag, h->unode, h->stamp, h->nbmask, h->flag, h->corner, h->bodyz,     h->dtypes,     h->x,          h->v,
                   h->fv,     h->vcell, h->vnode,     h->vtile,      h->cell_type,  h->cell_voff,
                   h->alive,  h->dcells_all, h->status, h->bin_counts, h->bin_cursor, h->bin_offsets,
                   h->tile_vertices, h->tile_cell_counts, h->tile_cell_offsets, h->tile_cells, h->scratch,
@@ -1833,7 +1837,35 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
                o_bo = put_i(c.bend_outer), o_ring = put_i(c.ring), o_rn = put_i(c.ring_n), o_in = put_i(c.inner),
                o_vf = put_i(c.vface), o_ve = put_i(c.vedge), o_vo = put_i(c.vopp), o_vio = put_i(c.vinner_off),
                o_vi = put_i(c.vinner), o_sr = put_i(c.slot_rot);
-  while (iv.size() % 2) iv.push_back(0);
+  // the packed tables (TypeDev), each from a 16-byte boundary
+  auto align16 = [&] {
+    while (iv.size() % 4) iv.push_back(0);
+    return iv.size();
+  };
+  auto put_six = [&](const std::vector<int>& a, bool ring) {
+    const size_t o = align16();
+    for (int i = 0; i < c.nv; ++i) {
+      uint32_t lane[8] = {};
+      for (int j = 0; j < c.ring_n[i]; ++j) {
+        lane[j] = (uint32_t)a[6 * i + j];
+        if (ring) lane[7] |= (uint32_t)c.slot_rot[6 * i + j] << (2 * j);
+      }
+      if (ring) lane[6] = (uint32_t)c.ring_n[i];
+      for (int w = 0; w < 4; ++w) iv.push_back((int)(lane[2 * w] | lane[2 * w + 1] << 16));
+    }
+    return o;
+  };
+  const bool narrow = c.nf < 65536 && c.ne < 65536;
+  const size_t o_r16 = put_six(c.ring, true), o_vf16 = narrow ? put_six(c.vface, false) : 0,
+               o_ve16 = narrow ? put_six(c.vedge, false) : 0, o_vo16 = narrow ? put_six(c.vopp, false) : 0,
+               o_t16 = align16();
+  for (int k = 0; k < c.nf; ++k) {
+    iv.push_back(c.tris[3 * k] | (int)((uint32_t)c.tris[3 * k + 1] << 16));
+    iv.push_back(c.tris[3 * k + 2]);
+  }
+  const size_t o_e16 = align16();
+  for (int e = 0; e < c.ne; ++e) iv.push_back(c.edges[2 * e] | (int)((uint32_t)c.edges[2 * e + 1] << 16));
+  align16();
   std::vector<double> dv;
   auto put_d = [&](const std::vector<double>& a) {
     size_t o = dv.size();
@@ -1845,7 +1877,7 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
   // the mixed form reads 32-bit copies, the plain form the reciprocals of the
   // rest areas and lengths
   std::vector<float> fv;
-  size_t o_ia = 0, o_iel = 0;
+  size_t o_ia = 0, o_iel = 0, o_sf = 0;
   if (h->f64) {
     auto reciprocals = [](std::vector<double> a) {
       for (double& x : a) x = 1.0 / x;
@@ -1855,7 +1887,14 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
     o_iel = put_d(reciprocals(c.edge_l0));
   } else {
     fv.assign(dv.begin(), dv.end());
+    while (fv.size() % 4) fv.push_back(0.f);
+    o_sf = fv.size();
+    for (int i = 0; i < c.nv; ++i) {
+      for (int j = 0; j < 6; ++j) fv.push_back((float)c.slot_a0[6 * i + j]);
+      for (int j = 0; j < 6; ++j) fv.push_back((float)c.slot_l0[6 * i + j]);
+    }
   }
+  if (dv.size() % 2) dv.push_back(0.0);  // the floats from a 16-byte boundary too
   const size_t ib = 4 * iv.size(), db = 8 * std::max<size_t>(dv.size(), 1), fb = 4 * std::max<size_t>(fv.size(), 1);
   HC_CUDA(h, dalloc(h, &ts.blob, ib + db + fb));
   HC_CUDA(h, cudaMemcpyAsync(ts.blob, iv.data(), ib, cudaMemcpyHostToDevice, h->stream));
@@ -1888,8 +1927,14 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
   d.slot_rot = ibase + o_sr;
   d.slot_a0 = dbase + o_sa;
   d.slot_l0 = dbase + o_sl;
-  d.slot_a0f = fbase + o_sa;
-  d.slot_l0f = fbase + o_sl;
+  auto six = [&](size_t o) { return narrow ? (const uint4*)(ibase + o) : nullptr; };
+  d.ring16 = (const uint4*)(ibase + o_r16);
+  d.vface16 = six(o_vf16);
+  d.vedge16 = six(o_ve16);
+  d.vopp16 = six(o_vo16);
+  d.tris16 = (const uint2*)(ibase + o_t16);
+  d.edges16 = (const uint32_t*)(ibase + o_e16);
+  d.slot_f = h->f64 ? nullptr : (const float4*)(fbase + o_sf);
   d.tri_a0 = dbase + o_a0;
   d.edge_l0 = dbase + o_l0;
   d.tri_ia0 = h->f64 ? dbase + o_ia : nullptr;
@@ -1903,7 +1948,9 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
   d.patch_d0f = fbase + o_pd;
   d.inner_l0f = fbase + o_il;
   d.volume_eq = c.volume_eq;
+  d.inv_volume_eq = 1.0 / c.volume_eq;
   d.area_mean_eq = c.area_mean_eq;
+  d.inv_area_mean_eq = 1.0 / c.area_mean_eq;
   d.edge_mean_eq = c.edge_mean_eq;
   d.k_link = ts.k.k_link;
   d.k_bend = ts.k.k_bend;

@@ -113,6 +113,22 @@ __device__ __forceinline__ void ld_cluster(uint32_t a, float& v) {
 __device__ __forceinline__ void ld_cluster(uint32_t a, double& v) {
   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
 }
+// the same from the CTA's own shared memory
+__device__ __forceinline__ void ld_shared(uint32_t a, float& v) {
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+}
+__device__ __forceinline__ void ld_shared(uint32_t a, double& v) {
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+}
+__device__ __forceinline__ void ld_shared4(uint32_t a, float* v) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+               : "r"(a));
+}
+__device__ __forceinline__ void ld_shared4(uint32_t a, double* v) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(a));
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[2]), "=d"(v[3]) : "r"(a + 16));
+}
 // four values from a 16-byte aligned address
 __device__ __forceinline__ void ld_cluster4(uint32_t a, float* v) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"

@@ -74,8 +74,11 @@ struct Kern {
   T w[8];
 };
 
-template <typename T>
-__device__ __forceinline__ void ibm_weights(const LbmView<T>& L, double px, double py, double pz, Kern<T>& K) {
+// load(nodes) is called with the node of every slot, skipped or not (0 off the
+// lattice), before the flags are waited for.
+template <typename T, typename Load>
+__device__ __forceinline__ void ibm_weights(const LbmView<T>& L, double px, double py, double pz, Kern<T>& K,
+                                            const Load& load) {
   constexpr bool kF64 = sizeof(T) == 8;
   const double P[3] = {px, py, pz};
   const int dims[3] = {L.nx, L.ny, L.nz};
@@ -139,27 +142,46 @@ __device__ __forceinline__ void ibm_weights(const LbmView<T>& L, double px, doub
       idx[a][k] = wrapped;
     }
   }
-  T total = T(0);
+  // the eight nodes' solid bits in one byte of the block's first node, in flight
+  // together with what else the caller loads per node (with eight scattered
+  // flags the FP32 force assembly of a 960-cell suspension took 134 us against
+  // 127; before, with the other loads waiting for them, 139)
+  uint32_t solid = 0;
+  if (idx[0][0] >= 0 && idx[1][0] >= 0 && idx[2][0] >= 0) {
+    const int base = idx[0][0] + L.nx * (idx[1][0] + L.ny * idx[2][0]);
+    solid = HC_IN(L.status, base, L.N) ? L.corner[base] : 0xffu;
+  } else {
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const int ax = s >> 2, ay = (s >> 1) & 1, az = s & 1;
+      if (idx[0][ax] < 0 || idx[1][ay] < 0 || idx[2][az] < 0) continue;
+      const int nd = idx[0][ax] + L.nx * (idx[1][ay] + L.ny * idx[2][az]);
+      if (!HC_IN(L.status, nd, L.N) || L.flag[nd] != 0) solid |= 1u << s;
+    }
+  }
   bool cut = false;  // a node that carries weight was left out
+  int nodes[8];
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
     const int ax = s >> 2, ay = (s >> 1) & 1, az = s & 1;
-    K.node[s] = -1;
-    K.w[s] = T(0);
-    if (idx[0][ax] < 0 || idx[1][ay] < 0 || idx[2][az] < 0) {
+    const bool off = idx[0][ax] < 0 || idx[1][ay] < 0 || idx[2][az] < 0;
+    const int nd = off ? 0 : idx[0][ax] + L.nx * (idx[1][ay] + L.ny * idx[2][az]);
+    const bool in = HC_IN(L.status, nd, L.N);
+    nodes[s] = in ? nd : 0;
+    cut |= off;
+    K.w[s] = phi[0][ax] * phi[1][ay] * phi[2][az];
+    K.node[s] = off || is_zero(K.w[s]) || !in ? -1 : nd;
+  }
+  load(nodes);
+  T total = T(0);
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    if (K.node[s] >= 0 && (solid >> s & 1u)) {
+      K.node[s] = -1;
       cut = true;
-      continue;
     }
-    const T w = phi[0][ax] * phi[1][ay] * phi[2][az];
-    if (is_zero(w)) continue;
-    const int nd = idx[0][ax] + L.nx * (idx[1][ay] + L.ny * idx[2][az]);
-    if (!HC_IN(L.status, nd, L.N) || L.flag[nd] != 0) {
-      cut = true;
-      continue;
-    }
-    if (!kF64) total += w;
-    K.node[s] = nd;
-    K.w[s] = w;
+    if (K.node[s] < 0) K.w[s] = T(0);
+    else if (!kF64) total += K.w[s];
   }
   // The weights of a whole stencil sum to one by themselves, to the rounding
   // of their products: FP64, whose pipe bounds the cell kernels, renormalises
@@ -173,6 +195,100 @@ __device__ __forceinline__ void ibm_weights(const LbmView<T>& L, double px, doub
 #pragma unroll
     for (int s = 0; s < 8; ++s) K.w[s] *= coeff;
   }
+}
+
+// Bit s of corner[n]: slot s of the 2x2x2 block from node n on is a boundary
+// node (unset beyond a non-periodic end, which the callers see themselves).
+__global__ void k_corner_flags(const uint8_t* flag, uint8_t* corner, int nx, int ny, int nz) {
+  const int X = blockIdx.x * blockDim.x + threadIdx.x;
+  if (X >= nx) return;
+  for (int Z = blockIdx.z; Z < nz; Z += gridDim.z)
+    for (int Y = blockIdx.y * blockDim.y + threadIdx.y; Y < ny; Y += gridDim.y * blockDim.y) {
+      uint32_t bits = 0;
+      for (int s = 0; s < 8; ++s) {
+        const int x = X + (s >> 2) < nx ? X + (s >> 2) : 0, y = Y + (s >> 1 & 1) < ny ? Y + (s >> 1 & 1) : 0,
+                  z = Z + (s & 1) < nz ? Z + (s & 1) : 0;
+        if (flag[x + (long long)nx * (y + (long long)ny * z)] != 0) bits |= 1u << s;
+      }
+      corner[X + (long long)nx * (Y + (long long)ny * Z)] = (uint8_t)bits;
+    }
+}
+cudaError_t launch_corner_flags(const uint8_t* flag, uint8_t* corner, int nx, int ny, int nz, cudaStream_t s) {
+  const dim3 block(32, 8), grid((nx + 31) / 32, std::min((ny + 7) / 8, 65535), std::min(nz, 65535));
+  k_corner_flags<<<grid, block, 0, s>>>(flag, corner, nx, ny, nz);
+  return cudaGetLastError();
+}
+
+template <typename T>
+__device__ __forceinline__ void ibm_weights(const LbmView<T>& L, double px, double py, double pz, Kern<T>& K) {
+  ibm_weights(L, px, py, pz, K, [](const int*) {});
+}
+// The velocity at (px, py, pz): the lower x-side's four nodes, then the upper's.
+template <typename T>
+__device__ __forceinline__ V3t<T> ibm_velocity(const LbmView<T>& L, double px, double py, double pz) {
+  Kern<T> K;
+  V3t<T> u[8], v[2] = {};
+  ibm_weights(L, px, py, pz, K, [&](const int* nd) {
+#pragma unroll
+    for (int s = 0; s < 8; ++s) FieldLayout<T>::load(L.unode, L.N, nd[s], u[s].x, u[s].y, u[s].z);
+  });
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (K.node[j] < 0) continue;
+    v[j >> 2].x += u[j].x * K.w[j];
+    v[j >> 2].y += u[j].y * K.w[j];
+    v[j >> 2].z += u[j].z * K.w[j];
+  }
+  return v[0] + v[1];
+}
+// Two neighbouring lanes share their stencils: of both vertices the even lane
+// takes the lower x-side (slots 0 to 3) and the odd lane the upper one, whose
+// nodes lie beside the lower's.  A load or atomic add of the warp then touches
+// 16 pairs of neighbouring nodes instead of 32 nodes of 32 vertices (27 lines of
+// 128 bytes for a turned red cell).  Force assembly of the 280-cell pipe: FP64
+// 184.7 us before, 179.1 now; FP32 39.1 and 37.7.  side[0..3] of the even lane's
+// vertex, side[4..7] of the odd lane's.
+template <typename V>
+__device__ __forceinline__ void pair_sides(const V own[8], V side[8]) {
+  const bool odd = threadIdx.x & 1;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const V other = __shfl_xor_sync(0xffffffffu, odd ? own[j] : own[4 + j], 1);
+    side[j] = odd ? other : own[j];
+    side[4 + j] = odd ? own[4 + j] : other;
+  }
+}
+// ibm_velocity by whole warps, the sums in the same order; a lane without a
+// vertex (on clear) takes part with weights of zero.
+template <typename T>
+__device__ __forceinline__ V3t<T> pair_velocity(const LbmView<T>& L, double px, double py, double pz, bool on) {
+  Kern<T> K;
+  V3t<T> u[8], v[2] = {};
+  ibm_weights(L, px, py, pz, K, [&](const int* own) {
+    int nd[8];
+    pair_sides(own, nd);
+#pragma unroll
+    for (int s = 0; s < 8; ++s) FieldLayout<T>::load(L.unode, L.N, nd[s], u[s].x, u[s].y, u[s].z);
+  });
+  T w[8];
+  if (!on) {
+#pragma unroll
+    for (int s = 0; s < 8; ++s) K.w[s] = T(0);
+  }
+  pair_sides(K.w, w);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (is_zero(w[j])) continue;
+    v[j >> 2].x += u[j].x * w[j];
+    v[j >> 2].y += u[j].y * w[j];
+    v[j >> 2].z += u[j].z * w[j];
+  }
+  // this lane's vertex is v[0] of an even lane, v[1] of an odd one
+  const bool odd = threadIdx.x & 1;
+  const V3t<T> own = odd ? v[1] : v[0], give = odd ? v[0] : v[1];
+  const V3t<T> other = {__shfl_xor_sync(0xffffffffu, give.x, 1), __shfl_xor_sync(0xffffffffu, give.y, 1),
+                        __shfl_xor_sync(0xffffffffu, give.z, 1)};
+  return own + other;
 }
 
 // ---------------------------------------------------------------------------
@@ -618,20 +734,10 @@ __global__ void __launch_bounds__(256) k_interp_advance(const LbmView<T> L, cons
   double px = vv.x[i], py = vv.x[V + i], pz = vv.x[2 * V + i];
   T vx, vy, vz;
   if (do_interp) {
-    Kern<T> K;
-    ibm_weights(L, px, py, pz, K);
-    vx = T(0);
-    vy = T(0);
-    vz = T(0);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (K.node[j] < 0) continue;
-      T ux, uy, uz;
-      FieldLayout<T>::load(L.unode, L.N, K.node[j], ux, uy, uz);
-      vx += ux * K.w[j];
-      vy += uy * K.w[j];
-      vz += uz * K.w[j];
-    }
+    const V3t<T> u = ibm_velocity(L, px, py, pz);
+    vx = u.x;
+    vy = u.y;
+    vz = u.z;
     vv.v[i] = vx;
     vv.v[V + i] = vy;
     vv.v[2 * V + i] = vz;
@@ -807,6 +913,14 @@ __device__ __forceinline__ V3t<T> ld3_cluster(uint32_t a) {
   ld_cluster(a + 2u * (uint32_t)sizeof(T), v.z);
   return v;
 }
+template <typename Terms, typename T>
+__device__ __forceinline__ V3t<T> ld3_terms(uint32_t a) {
+  V3t<T> v;
+  Terms::load(a, v.x);
+  Terms::load(a + (uint32_t)sizeof(T), v.y);
+  Terms::load(a + 2u * (uint32_t)sizeof(T), v.z);
+  return v;
+}
 // the sum of a double over the ranks, in their order: the same bits in each
 __device__ __forceinline__ double cluster_sum(const double* p, int cs) {
   double sum = 0.0;
@@ -820,18 +934,42 @@ __device__ __forceinline__ double cluster_sum(const double* p, int cs) {
 // Where item k of an array cut into chunks lies: its address in the owner's
 // shared memory.  magic = ceil(2^32 / chunk) makes the division exact for
 // k * chunk < 2^32 (at most 19,000 faces in chunks of at most that many).
+// ONE: the cell is one CTA's and every item its own.
+template <bool ONE>
 struct Chunked {
   uint32_t base, stride, magic;
   int chunk;
   __device__ __forceinline__ Chunked(const void* p, int chunk_, size_t stride_)
       : base(smem_addr(p)), stride((uint32_t)stride_), magic((uint32_t)((0x100000000ull + chunk_ - 1) / chunk_)),
         chunk(chunk_) {}
-  __device__ __forceinline__ uint32_t owner(int k) const { return __umulhi((uint32_t)k, magic); }
-  __device__ __forceinline__ uint32_t within(int k, uint32_t own) const { return (uint32_t)k - own * (uint32_t)chunk; }
+  __device__ __forceinline__ uint32_t owner(int k) const { return ONE ? 0u : __umulhi((uint32_t)k, magic); }
+  __device__ __forceinline__ uint32_t within(int k, uint32_t own) const {
+    return ONE ? (uint32_t)k : (uint32_t)k - own * (uint32_t)chunk;
+  }
   __device__ __forceinline__ uint32_t at(int k, uint32_t own) const {
-    return cluster_addr(base + within(k, own) * stride, own);
+    const uint32_t a = base + within(k, own) * stride;
+    return ONE ? a : cluster_addr(a, own);
   }
   __device__ __forceinline__ uint32_t at(int k) const { return at(k, owner(k)); }
+  template <typename T>
+  static __device__ __forceinline__ void load(uint32_t a, T& v) {
+    if constexpr (ONE) ld_shared(a, v);
+    else ld_cluster(a, v);
+  }
+  template <typename T>
+  static __device__ __forceinline__ void load4(uint32_t a, T* v) {
+    if constexpr (ONE) ld_shared4(a, v);
+    else ld_cluster4(a, v);
+  }
+};
+// six 16-bit indices in one 16-byte load (TypeDev)
+struct Six {
+  uint32_t w[4];
+  __device__ __forceinline__ Six(const uint4* table, int i) {
+    const uint4 v = table[i];
+    w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+  }
+  __device__ __forceinline__ int operator[](int j) const { return (int)(j & 1 ? w[j >> 1] >> 16 : w[j >> 1] & 0xffffu); }
 };
 
 // One CTA or cluster per cell (grid-stride over the cell list), vertex-centric: each
@@ -899,9 +1037,10 @@ __device__ __forceinline__ V3t<T> plt_bending(const T* sx, const TypeDev& t, int
 // just assembled (core/hemoCellParticleField.cpp:841-863): FORCE_LIMIT clamp
 // (the stored force stays unclamped, as after the reference's constitutive
 // model), plus the repulsion force, spread with the phi2 weights; the
-// stencil nodes are tagged for the interpolation.
+// stencil nodes are tagged for the interpolation.  By whole warps, two lanes to
+// a pair of vertices (pair_sides); a lane without a vertex (on clear) names any.
 template <typename T>
-__device__ __forceinline__ void spread_vertex(const MechView<T>& M, int gi, V3t<T> f) {
+__device__ __forceinline__ void spread_vertex(const MechView<T>& M, int gi, V3t<T> f, bool on) {
   const VertexView<T>& vv = M.vv;
   const long long V = vv.V;
   T mag = f.x * f.x;
@@ -918,11 +1057,24 @@ __device__ __forceinline__ void spread_vertex(const MechView<T>& M, int gi, V3t<
   ibm_weights(M.L, vv.x[gi], vv.x[V + gi], vv.x[2 * V + gi], K);
   const uint32_t stamp = *M.L.stamp + (M.fuse_advance ? 1u : 0u);
   T* F = const_cast<T*>(M.L.Fcur);
+  if (!on) {
+#pragma unroll
+    for (int s = 0; s < 8; ++s) K.node[s] = -1;
+  }
+  int node[8];
+  T w[8];
+  pair_sides(K.node, node);
+  pair_sides(K.w, w);
+  const V3t<T> other = {__shfl_xor_sync(0xffffffffu, f.x, 1), __shfl_xor_sync(0xffffffffu, f.y, 1),
+                        __shfl_xor_sync(0xffffffffu, f.z, 1)};
+  const bool odd = threadIdx.x & 1;
+  const V3t<T> even_f = odd ? other : f, odd_f = odd ? f : other;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    if (K.node[j] < 0) continue;
-    if (M.L.ntag) M.L.ntag[K.node[j]] = stamp;
-    FieldLayout<T>::add(F, M.L.N, K.node[j], f.x * K.w[j], f.y * K.w[j], f.z * K.w[j]);
+    if (node[j] < 0) continue;
+    const V3t<T> g = vscale(j < 4 ? even_f : odd_f, w[j]);
+    if (M.L.ntag) M.L.ntag[node[j]] = stamp;
+    FieldLayout<T>::add(F, M.L.N, node[j], g.x, g.y, g.z);
   }
 }
 
@@ -942,26 +1094,22 @@ __device__ __forceinline__ void advance_range(const MechView<T>& M, int voff, in
   const VertexView<T>& vv = M.vv;
   const LbmView<T>& L = M.L;
   const long long V = vv.V;
-  for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-    const int i = voff + k;
-    if (!alive) {
-      vv.vnode[i] = -1;
-      vv.vtile[i] = -1;
-      continue;
+  if (!alive) {
+    for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+      vv.vnode[voff + k] = -1;
+      vv.vtile[voff + k] = -1;
     }
+    return;
+  }
+  // whole warps, whose last one's spare lanes follow its last vertex
+  const int lane = threadIdx.x & 31;
+  for (int kw = k0 + (int)threadIdx.x - lane; kw < k1; kw += blockDim.x) {
+    const bool on = kw + lane < k1;
+    const int i = voff + min(kw + lane, k1 - 1);
     double px = vv.x[i], py = vv.x[V + i], pz = vv.x[2 * V + i];
-    Kern<T> K;
-    ibm_weights(L, px, py, pz, K);
-    T vx = T(0), vy = T(0), vz = T(0);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (K.node[j] < 0) continue;
-      T ux, uy, uz;
-      FieldLayout<T>::load(L.unode, L.N, K.node[j], ux, uy, uz);
-      vx += ux * K.w[j];
-      vy += uy * K.w[j];
-      vz += uz * K.w[j];
-    }
+    const V3t<T> u = pair_velocity(L, px, py, pz, on);
+    if (!on) continue;
+    const T vx = u.x, vy = u.y, vz = u.z;
     vv.v[i] = vx;
     vv.v[V + i] = vy;
     vv.v[2 * V + i] = vz;
@@ -999,6 +1147,21 @@ __device__ __forceinline__ void advance_range(const MechView<T>& M, int voff, in
     if (L.flag[nd] != 0) hit = 1;
   }
 }
+// the rest areas and lengths of vertex i's slots
+__device__ __forceinline__ void slot_rest(const TypeDev& t, int i, int, float a0[6], float l0[6]) {
+  const float4 p = t.slot_f[3 * i], q = t.slot_f[3 * i + 1], r = t.slot_f[3 * i + 2];
+  a0[0] = p.x, a0[1] = p.y, a0[2] = p.z, a0[3] = p.w, a0[4] = q.x, a0[5] = q.y;
+  l0[0] = q.z, l0[1] = q.w, l0[2] = r.x, l0[3] = r.y, l0[4] = r.z, l0[5] = r.w;
+}
+__device__ __forceinline__ void slot_rest(const TypeDev& t, int i, int rn, double a0[6], double l0[6]) {
+#pragma unroll
+  for (int j = 0; j < 6; ++j)
+    if (j < rn) {
+      a0[j] = t.slot_a0[6 * i + j];
+      l0[j] = t.slot_l0[6 * i + j];
+    }
+}
+
 // The vertex-centric force assembly of one cell's vertices [v0, v1) and faces
 // [f0, f1) by one rank of its cluster (variant 0; the staged variant falls back
 // to it for FP32 cell types whose terms would not share an SM).  sx holds
@@ -1017,7 +1180,7 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
   T* sbf = sx + 3 * nv;  // own bending force per own vertex
   uint8_t* srn = reinterpret_cast<uint8_t*>(sbf + 3 * vch);  // valence per vertex
   if (!HC_IN(vv.status, (long long)voff + nv - 1, V)) return;  // the cell's vertices in the arrays (every rank returns)
-  for (int k = tid; k < nv; k += bs) srn[k] = (uint8_t)t.ring_n[k];
+  for (int k = tid; k < nv; k += bs) srn[k] = (uint8_t)(t.ring16[k].w & 0xffffu);
   // positions relative to the cell's vertex 0 (translation invariant forces;
   // the volume sum stays well conditioned far from the origin)
   const double r0x = vv.x[voff], r0y = vv.x[V + voff], r0z = vv.x[2 * V + voff];
@@ -1038,7 +1201,8 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
   // --- phase 1: face volume terms, own bending force (rbcHighOrderModel.cpp:62-68, :127-157)
   double vol = 0.0;
   for (int k = f0 + tid; k < f1; k += bs) {
-    const V3t<T> v0 = ld3(sx, t.tris[3 * k]), v1 = ld3(sx, t.tris[3 * k + 1]), v2 = ld3(sx, t.tris[3 * k + 2]);
+    const uint2 c = t.tris16[k];
+    const V3t<T> v0 = ld3(sx, c.x & 0xffffu), v1 = ld3(sx, c.x >> 16), v2 = ld3(sx, c.y);
     if (kF64) {
       const double v210 = (double)v2.x * v1.y * v0.z, v120 = (double)v1.x * v2.y * v0.z;
       const double v201 = (double)v2.x * v0.y * v1.z, v021 = (double)v0.x * v2.y * v1.z;
@@ -1051,17 +1215,21 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
   }
   if (t.model != 1) {
     for (int i = v0 + tid; i < v1; i += bs) {
-      const int rn = t.ring_n[i];
-      const int* rg = t.ring + 6 * i;
+      const Six rg(t.ring16, i);
+      const int rn = rg[6];
       const V3t<T> xi = ld3(sx, i);
       V3t<T> sum = {T(0), T(0), T(0)};
-      for (int j = 0; j < rn; ++j) sum = sum + ld3(sx, rg[j]);
+#pragma unroll
+      for (int j = 0; j < 6; ++j)
+        if (j < rn) sum = sum + ld3(sx, rg[j]);
       const V3t<T> mid = {fdiv(sum.x, (T)rn), fdiv(sum.y, (T)rn), fdiv(sum.z, (T)rn)};
       const V3t<T> dev = mid - xi;
       V3t<T> pn = {T(0), T(0), T(0)};
       V3t<T> a = ld3(sx, rg[0]) - xi;
       const V3t<T> first = a;
-      for (int j = 0; j < rn; ++j) {
+#pragma unroll
+      for (int j = 0; j < 6; ++j) {
+        if (j >= rn) break;
         const V3t<T> b = (j + 1 < rn) ? ld3(sx, rg[j + 1]) - xi : first;
         T l;
         pn = pn + normalized(vcross(a, b), l);
@@ -1080,7 +1248,7 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
   }
   block_sum<T>(vol, red);  // red[32] = sum over the block
   cluster_sync(cs);
-  const Chunked bending(sbf, vch, 3 * sizeof(T));
+  const Chunked<false> bending(sbf, vch, 3 * sizeof(T));
   // volume constraint in FP64 (rbcHighOrderModel.cpp:100-104), by one thread
   if (tid == 0) {
     const double volume = cluster_sum(red + 32, cs) * (1.0 / 6.0);
@@ -1095,28 +1263,26 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
   const T area_mean = (T)t.area_mean_eq;
   const bool visc = (t.model != 0) || (t.eta_m != 0.0);
   // --- phase 2: gather per vertex
-  for (int i = v0 + tid; i < v1; i += bs) {
-    const int rn = t.ring_n[i];
+  for (int iw = v0 + (tid & ~31); iw < v1; iw += bs) {
+    // whole warps, whose last one's spare lanes repeat its last vertex
+    const int i = min(iw + (tid & 31), v1 - 1);
+    const bool on = iw + (tid & 31) < v1;
+    const Six rs(t.ring16, i);
+    const int rn = rs[6];
+    T a0s[6], l0s[6];
+    slot_rest(t, i, rn, a0s, l0s);
     const V3t<T> xi = ld3(sx, i);
     V3t<T> f = {T(0), T(0), T(0)};
     V3t<T> vi = {T(0), T(0), T(0)};
     if (visc) vi = {vv.v[voff + i], vv.v[V + voff + i], vv.v[2 * V + voff + i]};
-    int rs[6], rot[6];
-    T a0s[6], l0s[6];
+    int rot[6];
 #pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      if (j < rn) {
-        rs[j] = t.ring[6 * i + j];
-        rot[j] = t.slot_rot[6 * i + j];
-        a0s[j] = rest_value<T>(t.slot_a0, t.slot_a0f, 6 * i + j);
-        l0s[j] = rest_value<T>(t.slot_l0, t.slot_l0f, 6 * i + j);
-      }
-    }
+    for (int j = 0; j < 6; ++j) rot[j] = (rs[7] >> (2 * j)) & 3;
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
       if (j >= rn) break;
       const int r = rs[j];
-      const int r1 = rs[j + 1 < rn ? j + 1 : 0];
+      const int r1 = j + 1 < rn ? rs[j < 5 ? j + 1 : 0] : rs[0];
       // incident face (i, r, r1) in the reference's corner order: area force
       // on this corner and the face's volume force
       const V3t<T> xr = ld3(sx, r), xr1 = ld3(sx, r1);
@@ -1143,7 +1309,6 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
       if (kF64) f = f + vscale(vscale(F.n, vforce), F.area / area_mean);
       else f = f + vscale(F.n, vforce_per_area * F.area);
       // ring edge (i, r): link force toward r when stretched, viscosity
-      const int e = t.vedge[6 * i + j];
       T L;
       const V3t<T> uv = normalized(xr - xi, L);
       const T l0 = l0s[j];
@@ -1163,13 +1328,13 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
         f = f + V3t<T>{fdiv(-b.x, rnr), fdiv(-b.y, rnr), fdiv(-b.z, rnr)};
       } else {
         // platelet dihedral terms: end point of edge e, outer point of the opposite edge
-        f = f + plt_bending(sx, t, e);
+        f = f + plt_bending(sx, t, t.vedge[6 * i + j]);
         f = f - plt_bending(sx, t, t.vopp[6 * i + j]);
       }
     }
     if (t.model != 1) f = f + ld3(sbf, i - v0);
     // inner links (pltSimpleModel.cpp:188-205, wbcHighOrderModel.cpp:202-223)
-    for (int q = t.vinner_off[i]; q < t.vinner_off[i + 1]; ++q) {
+    for (int q = t.ni ? t.vinner_off[i] : 0, q1 = t.ni ? t.vinner_off[i + 1] : 0; q < q1; ++q) {
       const int e = t.vinner[q];
       const int o = t.inner[2 * e] == i ? t.inner[2 * e + 1] : t.inner[2 * e];
       const V3t<T> ev = ld3(sx, o) - xi;
@@ -1184,10 +1349,12 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
           f = f - vscale(vscale(uv, T(1) - L / (T(2) * (T)t.core_radius)), (T)t.k_inner_rigid);
       }
     }
-    vv.f[voff + i] = f.x;
-    vv.f[V + voff + i] = f.y;
-    vv.f[2 * V + voff + i] = f.z;
-    if (M.fuse_spread) spread_vertex(M, voff + i, f);
+    if (on) {
+      vv.f[voff + i] = f.x;
+      vv.f[V + voff + i] = f.y;
+      vv.f[2 * V + voff + i] = f.z;
+    }
+    if (M.fuse_spread) spread_vertex(M, voff + i, f, on);
   }
 }
 
@@ -1269,15 +1436,23 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 384 : 768) k_mechanics(const 
 // scalar along both of the corner's edges, so a vertex needs one scalar per
 // face and one per edge instead of two vectors.
 //
+// In FP32 latency bounds it: the chain of loads, barriers and reductions of one
+// cell, two cells an SM (more CTAs or threads an SM leave the first-level cache
+// too little room for the tables: 280 cells took 46 us, 52 to 59 with all of the
+// SM's memory shared).  So the tables are 16-bit, one load a vertex instead of
+// 18, and a cell on one CTA (ONE) reads its terms without a cluster's address
+// mapping: 45.6 to 41.9 us for the pipe, 152 to 139 for 960 cells.  Splitting
+// the last, nearly empty wave's cells over clusters made the latter 143.
+//
 // Shared layout after a header of 40 doubles: faces 4 words (cross product,
 // area scalar) and 1 word (inverse length of the cross product) of the own
-// chunk, positions 3 nv, own bending 3 vch, edge scalars ech, platelet dihedral
-// 3 ech (platelets only), valence nv bytes.
+// chunk, own bending 4 vch (force, 1/valence), edge scalars ech, platelet
+// dihedral 3 ech (platelets only), positions 3 nv.
 template <typename T>
 __host__ __device__ __forceinline__ size_t staged_smem_bytes(int model, int nv, int nf, int ne, int cluster) {
-  const size_t words = 5 * (size_t)cluster_chunk(nf, cluster) + 3 * (size_t)nv + 3 * (size_t)cluster_chunk(nv, cluster) +
+  const size_t words = 5 * (size_t)cluster_chunk(nf, cluster) + 4 * (size_t)cluster_chunk(nv, cluster) + 3 * (size_t)nv +
                        (size_t)cluster_chunk(ne, cluster) * (model == 1 ? 4 : 1);
-  return kClusterHeader * sizeof(double) + words * sizeof(T) + (size_t)nv;
+  return kClusterHeader * sizeof(double) + words * sizeof(T);
 }
 
 // x + x / |limit - x^2|, the saturating response of every membrane term
@@ -1301,13 +1476,13 @@ __device__ __forceinline__ T inv_valence(int n) {
 // a / b by a reciprocal: fast in both forms
 __device__ __forceinline__ float quotient(float a, float b) { return fdiv(a, b); }
 __device__ __forceinline__ double quotient(double a, double b) { return a * hcnewton::recip(b); }
-template <typename T>
-__global__ void __launch_bounds__(384) k_mechanics_staged(const MechView<T> M) {
+template <typename T, bool ONE>
+__global__ void __launch_bounds__(384, 2) k_mechanics_staged(const MechView<T> M) {
   extern __shared__ __align__(16) double smem_cluster[];
   __shared__ TypeDev t;
   __shared__ int hit;
   const int tid = threadIdx.x, bs = blockDim.x;
-  const int cs = (int)cluster_size(), rank = (int)cluster_rank();
+  const int cs = ONE ? 1 : (int)cluster_size(), rank = ONE ? 0 : (int)cluster_rank();
   const VertexView<T>& vv = M.vv;
   const long long V = vv.V;
   const int cell = M.cells[blockIdx.x / cs], voff = M.cell_voff[cell];
@@ -1321,11 +1496,10 @@ __global__ void __launch_bounds__(384) k_mechanics_staged(const MechView<T> M) {
   double* red = smem_cluster;
   T* sface = reinterpret_cast<T*>(smem_cluster + kClusterHeader);
   T* sinv = sface + 4 * fch;
-  T* sx = sinv + fch;
-  T* sbf = sx + 3 * nv;
-  T* sedge = sbf + 3 * vch;
+  T* sbf = sinv + fch;
+  T* sedge = sbf + 4 * vch;
   T* splt = sedge + ech;
-  uint8_t* srn = reinterpret_cast<uint8_t*>(splt + (plt ? 3 * ech : 0));
+  T* sx = splt + (plt ? 3 * ech : 0);
   if (!HC_IN(vv.status, (long long)voff + nv - 1, V)) alive = false;
   if (!alive) {
     for (int k = v0 + tid; k < v1; k += bs) {
@@ -1341,7 +1515,6 @@ __global__ void __launch_bounds__(384) k_mechanics_staged(const MechView<T> M) {
   // positions relative to the cell's vertex 0
   const double r0x = vv.x[voff], r0y = vv.x[V + voff], r0z = vv.x[2 * V + voff];
   for (int k = tid; k < nv; k += bs) {
-    srn[k] = (uint8_t)t.ring_n[k];
     sx[3 * k] = (T)(vv.x[voff + k] - r0x);
     sx[3 * k + 1] = (T)(vv.x[V + voff + k] - r0y);
     sx[3 * k + 2] = (T)(vv.x[2 * V + voff + k] - r0z);
@@ -1350,7 +1523,8 @@ __global__ void __launch_bounds__(384) k_mechanics_staged(const MechView<T> M) {
   // --- own faces: six times the signed volume, area force, cross product
   double vol = 0.0;
   for (int k = f0 + tid; k < f1; k += bs) {
-    const V3t<T> a = ld3(sx, t.tris[3 * k]), b = ld3(sx, t.tris[3 * k + 1]), c = ld3(sx, t.tris[3 * k + 2]);
+    const uint2 corner = t.tris16[k];
+    const V3t<T> a = ld3(sx, corner.x & 0xffffu), b = ld3(sx, corner.x >> 16), c = ld3(sx, corner.y);
     const V3t<T> n = vcross(b - a, c - a);
     vol += (double)vdot(a, n);
     T inv, len;
@@ -1365,7 +1539,8 @@ __global__ void __launch_bounds__(384) k_mechanics_staged(const MechView<T> M) {
   }
   // --- own edges: link and viscous force per edge vector, dihedral force
   for (int e = e0 + tid; e < e1; e += bs) {
-    const int a = t.edges[2 * e], b = t.edges[2 * e + 1];
+    const uint32_t ends = t.edges16[e];
+    const int a = (int)(ends & 0xffffu), b = (int)(ends >> 16);
     const V3t<T> d = ld3(sx, b) - ld3(sx, a);
     T inv, len;
     hcnewton::inv_length(vdot(d, d), inv, len);
@@ -1389,80 +1564,107 @@ __global__ void __launch_bounds__(384) k_mechanics_staged(const MechView<T> M) {
   }
   block_sum<T>(vol, red);  // red[32] = the own faces' sum
   cluster_sync(cs);
-  const Chunked faces(sface, fch, 4 * sizeof(T)), edges(sedge, ech, sizeof(T)), dihedral(splt, ech, 3 * sizeof(T)),
-      bending(sbf, vch, 3 * sizeof(T));
+  using Terms = Chunked<ONE>;
+  const Terms faces(sface, fch, 4 * sizeof(T)), edges(sedge, ech, sizeof(T)), dihedral(splt, ech, 3 * sizeof(T)),
+      bending(sbf, vch, 4 * sizeof(T));
   const uint32_t inv_base = smem_addr(sinv);
   // --- volume constraint in FP64, by one thread of each rank, over the ranks'
-  // sums in their order (the same bits in every rank)
+  // sums in their order (the same bits in every rank); its warp's bending waits
+  // for it, so there are no divisions in it (960 FP32 cells 127 us with, 122
+  // without)
   if (tid == 0) {
-    const double vfr = (cluster_sum(red + 32, cs) * (1.0 / 6.0) - t.volume_eq) / t.volume_eq;
-    red[33] = -t.k_volume * vfr / fabs(kMaxVol - vfr * vfr) / t.area_mean_eq;
+    const double sum = ONE ? red[32] : cluster_sum(red + 32, cs);
+    const double vfr = (sum * (1.0 / 6.0) - t.volume_eq) * t.inv_volume_eq;
+    red[33] = -t.k_volume * vfr * hcnewton::recip(fabs(kMaxVol - vfr * vfr)) * t.inv_area_mean_eq;
   }
   // --- own bending forces, from the unit normals of the incident faces
   if (!plt) {
     for (int i = v0 + tid; i < v1; i += bs) {
-      const int rn = srn[i];
+      const Six ring(t.ring16, i), face(t.vface16, i);
+      const int rn = ring[6];
       V3t<T> sum = {T(0), T(0), T(0)}, pn = {T(0), T(0), T(0)};
 #pragma unroll
       for (int j = 0; j < 6; ++j) {
         if (j >= rn) break;
-        sum = sum + ld3(sx, t.ring[6 * i + j]);
-        const int k = t.vface[6 * i + j];
+        sum = sum + ld3(sx, ring[j]);
+        const int k = face[j];
         const uint32_t owner = faces.owner(k);
         T q[4], s;
-        ld_cluster4(faces.at(k, owner), q);
-        ld_cluster(cluster_addr(inv_base + (uint32_t)sizeof(T) * faces.within(k, owner), owner), s);
+        Terms::load4(faces.at(k, owner), q);
+        const uint32_t at = inv_base + (uint32_t)sizeof(T) * faces.within(k, owner);
+        Terms::load(ONE ? at : cluster_addr(at, owner), s);
         pn = pn + vscale(V3t<T>{q[0], q[1], q[2]}, s);
       }
       T inv, len;
       hcnewton::inv_length(vdot(pn, pn), inv, len);
-      const V3t<T> dev = vscale(sum, inv_valence<T>(rn)) - ld3(sx, i);
+      // the mean's last place decides the deviation's fourth: in FP32 divided as
+      // in the vertex-centric kernel, so that both agree
+      const T part = inv_valence<T>(rn);
+      V3t<T> dev = vscale(sum, part);
+      if constexpr (sizeof(T) == 4) dev = {fdiv(sum.x, (T)rn), fdiv(sum.y, (T)rn), fdiv(sum.z, (T)rn)};
+      dev = dev - ld3(sx, i);
       pn = vscale(pn, inv);
       const T d = quotient(vdot(pn, dev) - rest_value<T>(t.patch_d0, t.patch_d0f, i), (T)t.edge_mean_eq);
       const T s = (T)t.k_bend * saturating(d, T(kMaxBend));
-      T* q = sbf + 3 * (i - v0);
+      T* q = sbf + 4 * (i - v0);
       q[0] = pn.x * s;
       q[1] = pn.y * s;
       q[2] = pn.z * s;
+      q[3] = part;
     }
   }
   cluster_sync(cs);
   const T push = T(0.5) * (T)red[33];  // volume force per cross product
   // --- gather the own vertices' forces
-  for (int i = v0 + tid; i < v1; i += bs) {
-    const int rn = srn[i];
+  for (int iw = v0 + (tid & ~31); iw < v1; iw += bs) {
+    // whole warps, whose last one's spare lanes repeat its last vertex
+    const int i = min(iw + (tid & 31), v1 - 1);
+    const bool on = iw + (tid & 31) < v1;
+    const Six ring(t.ring16, i), face(t.vface16, i), edge(t.vedge16, i), opp(plt ? t.vopp16 : t.vedge16, i);
+    const int rn = ring[6];
     const V3t<T> xi = ld3(sx, i);
     V3t<T> f = {T(0), T(0), T(0)}, n = {T(0), T(0), T(0)};
     T af[6], last = T(0);
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
       if (j >= rn) break;
-      const int k = t.vface[6 * i + j];
       T q[4];
-      ld_cluster4(faces.at(k, faces.owner(k)), q);
+      Terms::load4(faces.at(face[j]), q);
       n = n + V3t<T>{q[0], q[1], q[2]};
       af[j] = last = q[3];
     }
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
       if (j >= rn) break;
-      const int r = t.ring[6 * i + j], e = t.vedge[6 * i + j];
+      const int r = ring[j], e = edge[j];
       T pull;
-      ld_cluster(edges.at(e), pull);
+      Terms::load(edges.at(e), pull);
       // the edge's own scalar and a third of its two faces'
       const T c = pull + T(1.0 / 3.0) * (af[j] + (j == 0 ? last : af[j - 1]));
       f = f + vscale(ld3(sx, r) - xi, c);
-      if (!plt) f = f - vscale(ld3_cluster<T>(bending.at(r)), inv_valence<T>(srn[r]));
-      else f = f + ld3_cluster<T>(dihedral.at(e)) - ld3_cluster<T>(dihedral.at(t.vopp[6 * i + j]));
+      if (!plt) {
+        T q[4];
+        Terms::load4(bending.at(r), q);
+        f = f - vscale(V3t<T>{q[0], q[1], q[2]}, q[3]);
+      } else {
+        f = f + ld3_terms<Terms, T>(dihedral.at(e)) - ld3_terms<Terms, T>(dihedral.at(opp[j]));
+      }
     }
     f = f + vscale(n, push);
-    if (!plt) f = f + ld3(sbf, i - v0);
-    for (int q = t.vinner_off[i]; q < t.vinner_off[i + 1]; ++q) {
+    if (!plt) f = f + V3t<T>{sbf[4 * (i - v0)], sbf[4 * (i - v0) + 1], sbf[4 * (i - v0) + 2]};
+    for (int q = t.ni ? t.vinner_off[i] : 0, q1 = t.ni ? t.vinner_off[i + 1] : 0; q < q1; ++q) {
       const int e = t.vinner[q];
       const int o = t.inner[2 * e] == i ? t.inner[2 * e + 1] : t.inner[2 * e];
       const V3t<T> ev = ld3(sx, o) - xi;
       T inv, len;
-      hcnewton::inv_length(vdot(ev, ev), inv, len);
+      if constexpr (sizeof(T) == 8) {
+        hcnewton::inv_length(vdot(ev, ev), inv, len);
+      } else {
+        // the strain is the difference of nearly equal lengths: the rounded root,
+        // as in the vertex-centric kernel
+        len = vnorm(ev);
+        inv = T(1) / len;
+      }
       const V3t<T> uv = vscale(ev, inv);  // toward the partner
       if (plt) {
         const T l0 = rest_value<T>(t.inner_l0, t.inner_l0f, e);
@@ -1473,10 +1675,12 @@ __global__ void __launch_bounds__(384) k_mechanics_staged(const MechView<T> M) {
         if (len < d2) f = f - vscale(uv, (T(1) - quotient(len, d2)) * (T)t.k_inner_rigid);
       }
     }
-    vv.f[voff + i] = f.x;
-    vv.f[V + voff + i] = f.y;
-    vv.f[2 * V + voff + i] = f.z;
-    if (M.fuse_spread) spread_vertex(M, voff + i, f);
+    if (on) {
+      vv.f[voff + i] = f.x;
+      vv.f[V + voff + i] = f.y;
+      vv.f[2 * V + voff + i] = f.z;
+    }
+    if (M.fuse_spread) spread_vertex(M, voff + i, f, on);
   }
   cluster_sync(cs);  // no rank leaves while another reads its terms
   end_launch(M);
@@ -1485,7 +1689,7 @@ __global__ void __launch_bounds__(384) k_mechanics_staged(const MechView<T> M) {
 template <typename T>
 cudaError_t launch_mechanics_staged(const MechView<T>& M, int cluster, int bs, cudaStream_t s) {
   if (M.ncells <= 0) return cudaSuccess;
-  return launch_cluster(k_mechanics_staged<T>, cluster, dim3(M.ncells * cluster), dim3(bs), M.dyn_smem, s, M.L.pdl,
+  return launch_cluster(cluster == 1 ? k_mechanics_staged<T, true> : k_mechanics_staged<T, false>, cluster, dim3(M.ncells * cluster), dim3(bs), M.dyn_smem, s, M.L.pdl,
                         M.carveout, M);
 }
 size_t mechanics_staged_bytes(int model, int nv, int nf, int ne, int cluster, bool f64) {
@@ -1707,19 +1911,20 @@ cudaError_t prepare_mechanics(int smem_bytes, int* staged_limit) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
-  void (*kernels[3])(const MechView<T>) = {k_mechanics<T>, k_mechanics_scatter<T>, k_mechanics_staged<T>};
-  for (int k = 0; k < 3; ++k) {
+  void (*kernels[4])(const MechView<T>) = {k_mechanics<T>, k_mechanics_scatter<T>, k_mechanics_staged<T, true>,
+                                           k_mechanics_staged<T, false>};
+  for (int k = 0; k < 4; ++k) {
     cudaFuncAttributes a;
     if ((e = cudaFuncGetAttributes(&a, kernels[k])) != cudaSuccess) return e;
     const int room = optin - (int)a.sharedSizeBytes;
     if (k < 2 && smem_bytes > room) return cudaErrorInvalidValue;
     e = cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize, room);
     if (e != cudaSuccess) return e;
-    if (k == 2) *staged_limit = room;
+    if (k >= 2) *staged_limit = k == 2 ? room : std::min(*staged_limit, room);
   }
   e = cudaFuncSetAttribute(k_mechanics<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_mechanics_staged<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return cudaFuncSetAttribute(k_mechanics_staged<T, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
 template <typename T>
@@ -1735,7 +1940,7 @@ bool mechanics_cluster_fits(bool staged, int cluster, int bs, int smem_bytes) {
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, staged ? k_mechanics_staged<T> : k_mechanics<T>, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, staged ? k_mechanics_staged<T, false> : k_mechanics<T>, &cfg) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

@@ -51,6 +51,7 @@ struct LbmView {
   T* __restrict__ Fnext;
   const uint32_t* __restrict__ nbmask;
   const uint8_t* __restrict__ flag;
+  const uint8_t* __restrict__ corner;  // solid bits of each node's 2x2x2 block (k_corner_flags)
   const T* __restrict__ bodyz;  // [3][nz]
   uint32_t* ntag;                // per node: stamp of the last step whose stencils touch it; null
                                  // when the node-velocity form in use evaluates every fluid node
@@ -134,8 +135,17 @@ struct TypeDev {
   const int* slot_rot;    // nv*6
   const double* slot_a0;  // nv*6
   const double* slot_l0;  // nv*6
-  const float* slot_a0f;
-  const float* slot_l0f;
+  // The same tables in 16-bit indices, one 16-byte load a vertex (lane j of six;
+  // the ring's lanes 6 and 7 hold ring_n and slot_rot in two bits each), one
+  // 8-byte load a face and one 4-byte load an edge.  vface16 and later need
+  // nf, ne < 65536 (null otherwise).
+  const uint4* ring16;
+  const uint4* vface16;
+  const uint4* vedge16;
+  const uint4* vopp16;
+  const uint2* tris16;
+  const uint32_t* edges16;
+  const float4* slot_f;  // per vertex 6 slot_a0, then 6 slot_l0 (FP32 handles only)
   const double* tri_a0;
   const double* edge_l0;
   const double* tri_ia0;  // reciprocals of tri_a0 and edge_l0 (FP64 handles only)
@@ -149,6 +159,7 @@ struct TypeDev {
   const float* patch_d0f;
   const float* inner_l0f;
   double volume_eq, area_mean_eq, edge_mean_eq;
+  double inv_volume_eq, inv_area_mean_eq;  // reciprocals
   double k_link, k_bend, k_volume, k_area, eta_m, k_inner_rigid, k_cyto, core_radius, radius;
 };
 
@@ -315,6 +326,7 @@ cudaError_t launch_convert_in(const double* src, T* dst, long long n, cudaStream
 // hc_cells.cu
 template <typename T>
 cudaError_t launch_spread(const LbmView<T>& L, const VertexView<T>& vv, double f_limit, int bs, cudaStream_t s);
+cudaError_t launch_corner_flags(const uint8_t* flag, uint8_t* corner, int nx, int ny, int nz, cudaStream_t s);
 template <typename T>
 cudaError_t launch_mark_nodes(const LbmView<T>& L, const VertexView<T>& vv, cudaStream_t s);
 template <typename T>
