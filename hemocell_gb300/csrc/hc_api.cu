@@ -371,16 +371,18 @@ VertexView<T> vertex_view(hc_handle* h) {
 //   node costs the issue slots as much as a full one (pipe 64x64x256 82 against
 //   110 for the kernel, 150^3 Couette box 338 against 384).
 //   In FP32: (x, y)-blocks, or the list where rows rounded up to warps idle a
-//   twentieth of their lanes (rows of 64: 92 against 96; of 97: 29 against 32; of
-//   181: 65 against 67); evict-last population stores (pipe 92 against 96,
-//   suspension 128^3 241 against 244, elsewhere within 1%).
+//   twentieth of their lanes (pipe, rows of 64: 84 against 89; of 97: 29 against
+//   32; of 181: 65 against 67).  Evict-last population stores while both buffers
+//   take at most half the L2 (61x59x131 pipe with repulsion 22.4 against 22.9 ms
+//   for 400 steps); beyond it they cost (pipe 83.5 against 82.2, the 181x117x93
+//   channel 65.7 against 63.6, the 128^3 suspension the same 212).
 //   Node velocity in FP32: every fluid node from one vertex for 24 nodes on (96^3
-//   with 80 RBCs 78 against 81; with 20 65 against 72 the other way), else the
+//   with 80 RBCs 71 against 72; with 20 60 against 68 the other way), else the
 //   tagged nodes packed into warps from half a million nodes on (128^3 with 6
-//   RBCs 96 against 101; 64^3 with 8 36.9 against 35.8).  In FP64 tagged fluid
-//   nodes (pipe 294; every node 297, packed 297; 50^3 box 58, 66, 60).
-//   Programmatic launch always (32^3 box 28.7 against 30.5; FP64 50^3 box 82
-//   against 94).
+//   RBCs 90 against 97; 64^3 with 8 the same 32).  In FP64 tagged fluid nodes
+//   (50^3 box 56; every node 62, packed 58; pipe 289, 295, 287).
+//   Programmatic launch always (FP64 50^3 box 56 against 67, FP32 32^3 box 25.6
+//   against 25.7).
 //   Force assembly: variant 2 (see mech_plan).
 void apply_rules(hc_handle* h) {
   if (h->tuned) return;
@@ -398,7 +400,7 @@ void apply_rules(hc_handle* h) {
     return;
   }
   if (!fast32) return;
-  h->tune[7] |= 0x2000;
+  if (h->nfluid > 0 && 152LL * h->nfluid <= 64 << 20) h->tune[7] |= 0x2000;
   if (24LL * h->nvert >= h->N) h->tune[7] |= 0x300;
   else if (h->N >= 500000) h->tune[7] |= 0x200;
 }
@@ -793,7 +795,7 @@ size_t gather_bytes(const hc_handle* h, const TypeSlot& ts, int cluster = 1) {
 // own, at most 8.  FP64, whose one pipe an SM bounds it, splits finer, so that
 // the SMs' shares come out even and one CTA's loads fill another's gaps: 2 at
 // least, 4 up to three CTAs an SM (two where other types' CTAs need room beside
-// them: 110 RBCs with 11 platelets and a WBC take 162 us a step on 4 CTAs a
+// them: 110 RBCs with 11 platelets and a WBC took 162 us a step on 4 CTAs a
 // cell, some of which then wait for a second wave), 8 up to two.  Either form takes 16 where 8
 // would leave a CTA more than 96 vertices.  The kernel in microseconds, staged,
 // with the advance and spread in it, n RBCs of 642 vertices on 1 / 2 / 4 / 8 CTAs
@@ -897,8 +899,9 @@ int enq_types(hc_handle* h, hcd::MechView<T> M, bool forced, bool all_due) {
     M.before_next = overlap && k + 1 < launches.size();
     M.L.pdl = pdl || M.after_prev;
     // an SM configured for small CTAs takes no large one until they end: side by
-    // side all launches run on the same split of the SM's memory (an FP64
-    // suspension's step 222 us against 247 without, 232 at 100 percent)
+    // side all launches run on the same split of the SM's memory (FP32 128^3
+    // suspension 212 us a step against 224 without, 220 at 100 percent; FP64
+    // 67x81x50 suspension 140.5, 140.5, 147)
     M.carveout = overlap ? 55 : 0;
     if (l.plan.staged) HC_CUDA(h, hcd::launch_mechanics_staged<T>(M, l.plan.cluster, l.plan.bs, h->stream));
     else HC_CUDA(h, hcd::launch_mechanics<T>(M, l.plan.cluster, l.plan.bs, 0, h->tune[6] == 1 ? 1 : 0, h->stream));
