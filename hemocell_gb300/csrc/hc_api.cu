@@ -2441,15 +2441,18 @@ long long hc_estimate_device_bytes(const hc_params* p, int nvertices, int ncells
   const long long fb = 19 * ts * N;
   const long long Fb = (long long)(f64 ? hcd::field_bytes<double>(N) : hcd::field_bytes<float>(N));
   // lattice arrays, as hc_create allocates them
-  long long b = 2 * fb + 2 * Fb + 4 * N + Fb + 4 + 4 * N + N + 3 * ts * p->nz +
+  long long b = 2 * fb + 2 * Fb + 4 * N + Fb + 4 + 4 * N + 2 * N + 3 * ts * p->nz +
                 (long long)sizeof(TypeDev) * hcd::MAX_TYPES + 4;
   b += 4 * N;  // the fluid-node list (at most every node)
   // vertex and cell arrays at the capacity growth can reach (twice the need)
   const long long vcap = std::max<long long>(2LL * nvertices, 1024);
   const long long ccap = std::max<long long>(2LL * ncells, 64);
   b += vcap * (3 * 8 + 6 * ts + 3 * 4) + ccap * 4 * 4;
-  // per-type rest-state blobs and cell lists: at most ~512 bytes per vertex
-  b += 512LL * nvertices + 4LL * ncells;
+  // per-type rest-state blobs (hc_add_cell_type) and cell lists.  A closed mesh
+  // has 2 faces and 3 edges a vertex, at most one inner link for two vertices:
+  // 81 ints, 21.5 doubles, and 5 doubles or 33.5 floats more; 16-byte alignment
+  // of the tables within a blob
+  b += (f64 ? 536LL : 630LL) * nvertices + 128LL * hcd::MAX_TYPES + 4LL * ncells;
   // tile lists (hc_read_bins) and readback staging (hc_read_fluid, hc_read_vertices)
   const int tx = p->tile[0] > 0 ? p->tile[0] : 8, ty = p->tile[1] > 0 ? p->tile[1] : 8,
             tz = p->tile[2] > 0 ? p->tile[2] : 8;
