@@ -99,7 +99,7 @@ HC_POS_HD double from_fixed(int64_t x, int top) {
 // units small enough for every later exponent to stay normal
 constexpr int kLeastTop = 200;
 constexpr int kVelocityTop = 1016;   // u in units of 2^-64, |u| < 1/4
-constexpr int kRelaxationTop = 1017;  // 1 - omega in units of 2^-63
+constexpr int kRelaxationTop = 1018;  // 1 - omega, which rounds to 1 for a large tau, in units of 2^-62
 
 // The common exponent of the populations and the force; 2047 when one of them
 // is not finite.
@@ -143,7 +143,7 @@ struct Relax {
   double om, gF;  // omega, -3 (1 - omega/2)
   double am, aF;  // omega 4.5/36 and (1 - omega/2) 9/36
   double bm, bF;  // omega 3/36 and (1 - omega/2) 3/36
-  int64_t om1;    // 1 - omega in units of 2^-63
+  int64_t om1;    // 1 - omega in units of 2^-62
 };
 inline Relax relax_constants(double om) {
   const double hs = 1.0 - 0.5 * om;
@@ -188,7 +188,7 @@ HC_POS_HD bool collide(const double f[19], double Fx, double Fy, double Fz, cons
   int64_t left = M.mass;
   auto pair = [&](int i, int64_t cu, int64_t ca, int64_t cb, int64_t p) {
     const int64_t e = p + mul_high(cu, ca);
-    const int64_t plus = mul_high(2 * x[i + 9], k.om1) + e + cb, minus = mul_high(2 * x[i], k.om1) + e - cb;
+    const int64_t plus = mul_high(4 * x[i + 9], k.om1) + e + cb, minus = mul_high(4 * x[i], k.om1) + e - cb;
     left -= plus + minus;
     store(i + 9, from_fixed(plus, top));
     store(i, from_fixed(minus, top));
