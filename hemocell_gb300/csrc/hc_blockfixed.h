@@ -5,11 +5,14 @@
 // while its 32-bit integer units issue four warp instructions a cycle.  A node's
 // 19 populations and its force share one exponent, that of the largest of them:
 // each becomes a 64-bit integer in units of 2^(top - 57), where 2^top is at most
-// the largest magnitude.  That keeps 58 bits of the largest value, five more than
-// a double, so sums are exact, and what a conversion drops is at most a thirty-second
-// of the largest value's last place.  Sums, the pair terms and the relaxation run
-// on those integers; the dozen scalars of a node (1/rho, u, the vectors a and b)
-// stay in FP64: 36 FP64 instructions a node instead of 143.
+// the largest magnitude.  All of them are then held to half such a unit: 58 bits of
+// the largest, as many fewer of a smaller one as it is smaller (below a 32nd of the
+// largest fewer than a double's 53), and sums are exact.  Double arithmetic, whose
+// moments round to 2^-53 of the largest and enter every population, is no closer:
+// whole runs are a tenth as far off (tests/lattice_error_check.cpp).  Sums, the pair
+// terms and the relaxation run on those integers; the scalars of a node (1/rho, u,
+// the even part, the force's shares) stay in FP64: 30 FP64 instructions a node
+// instead of 143.
 //
 // Bounds: |v| < 2^(top + 1) for every population and force component, so the
 // moments stay below 19, a below 6, b below 4 and the results below 25 of those
@@ -120,7 +123,7 @@ HC_POS_HD int block_top(const double f[19], double Fx, double Fy, double Fz) {
 }
 
 struct Moments {
-  int64_t mass;  // rhoBar in units
+  int64_t mass, Jx, Jy, Jz;  // rhoBar and j in units
   double rhoBar, jx, jy, jz;
 };
 HC_POS_HD Moments fixed_moments(const int64_t x[19], int top) {
@@ -135,19 +138,37 @@ HC_POS_HD Moments fixed_moments(const int64_t x[19], int top) {
   const int64_t r = x[0] + ((p[1] + p[2]) + (p[3] + p[4])) + ((p[5] + p[6]) + (p[7] + p[8])) + p[9];
   const int64_t jx = (d[1] + d[4]) + (d[5] + d[6]) + d[7], jy = (d[2] + d[4]) - d[5] + (d[8] + d[9]),
                 jz = (d[3] + d[6]) - d[7] + (d[8] - d[9]);
-  return {r, from_fixed(r, top), from_fixed(jx, top), from_fixed(jy, top), from_fixed(jz, top)};
+  return {r, jx, jy, jz, from_fixed(r, top), from_fixed(jx, top), from_fixed(jy, top), from_fixed(jz, top)};
 }
 
 // omega-dependent constants of the collision (see hcd::CollideK)
 struct Relax {
-  double om, gF;  // omega, -3 (1 - omega/2)
-  double am, aF;  // omega 4.5/36 and (1 - omega/2) 9/36
-  double bm, bF;  // omega 3/36 and (1 - omega/2) 3/36
-  int64_t om1;    // 1 - omega in units of 2^-62
+  double om, gF, aF;  // omega, -3 (1 - omega/2), (1 - omega/2) / 8
+  int32_t bhi, blo;   // omega 3/36 in units of 2^-63: bhi 2^31 + blo, blo >= 0
+  int64_t om1;        // 1 - omega in units of 2^-62
 };
+// omega / 12 in units of 2^-63, to the nearest: omega = m 2^(e - 53) with a whole m
+inline int64_t omega_twelfth(double om) {
+  int e;
+  const uint64_t m = (uint64_t)ldexp(frexp(om, &e), 53);
+  const int up = 10 + e;
+  if (up <= -64) return 0;
+  return (int64_t)(((up >= 0 ? (unsigned __int128)m << up : (unsigned __int128)(m >> -up)) + 6) / 12);
+}
+// J omega / 12 to the nearest, |J| < 2^62: with J = j1 2^32 + j0 the quotient
+// (j1 2^32 + j0) (bhi 2^31 + blo) / 2^63 takes four 32-bit products
+HC_POS_HD int64_t momentum_share(int64_t J, const Relax& k) {
+  const int32_t j1 = (int32_t)(J >> 32);
+  const uint32_t j0 = (uint32_t)J;
+  const int64_t low = (int64_t)j1 * k.blo + (int64_t)(((uint64_t)j0 * (uint32_t)k.blo >> 32) + (1u << 30));
+  const int64_t mid = (int64_t)((uint64_t)low << 1) + (int64_t)((uint64_t)j0 * (uint32_t)k.bhi);
+  return (int64_t)j1 * k.bhi + (mid >> 32);
+}
 inline Relax relax_constants(double om) {
   const double hs = 1.0 - 0.5 * om;
-  return {om, -3.0 * hs, 0.125 * om, 0.25 * hs, om / 12.0, hs / 12.0, to_fixed(1.0 - om, kRelaxationTop)};
+  const int64_t b = omega_twelfth(om);
+  return {om, -3.0 * hs, 0.125 * hs, (int32_t)(b >> 31), (int32_t)(b & 0x7fffffff),
+          to_fixed(1.0 - om, kRelaxationTop)};
 }
 
 // The Guo-forced BGK collision of the pair terms P + Q, P - Q (see
@@ -177,14 +198,21 @@ HC_POS_HD bool collide(const double f[19], double Fx, double Fy, double Fz, cons
   // rounding down
   const int64_t P4 = to_fixed(even * (1.0 / 9.0), top) + 4;
   const int64_t P2 = (P4 - 1) >> 1, P = P4 >> 2, Q = (P4 + 2) >> 2;
-  const int64_t ax = to_fixed(fma(k.am, mx, k.aF * Fx), top), ay = to_fixed(fma(k.am, my, k.aF * Fy), top),
-                az = to_fixed(fma(k.am, mz, k.aF * Fz), top);
-  const int64_t bx = to_fixed(fma(k.bm, mx, k.bF * Fx), top), by = to_fixed(fma(k.bm, my, k.bF * Fy), top),
-                bz = to_fixed(fma(k.bm, mz, k.bF * Fz), top);
+  // b = w (3 omega m + 3 (1 - omega/2) F) = omega/12 j + F/12 with j in whole units:
+  // a factor omega/12 of 53 bits gave or took the same 1e-16 of the momentum in
+  // every step, and the velocities drifted: a quarter of the set-ups of
+  // tests/lattice_error_check.cpp were up to 1.3 times as far off as FP64, of
+  // which none is half as far now.  a = w (4.5 omega m + 9 (1 - omega/2) F) is 3/2
+  // of it and F (1 - omega/2) / 8.
+  auto share = [&](int64_t J, double F) { return momentum_share(J, k) + to_fixed(F * (1.0 / 12.0), top); };
+  auto forced = [&](int64_t b, double F) { return b + (b >> 1) + to_fixed(k.aF * F, top); };
+  const int64_t bx = share(M.Jx, Fx), by = share(M.Jy, Fy), bz = share(M.Jz, Fz);
+  const int64_t ax = forced(bx, Fx), ay = forced(by, Fy), az = forced(bz, Fz);
   const int64_t vx = to_fixed(ux, kVelocityTop), vy = to_fixed(uy, kVelocityTop), vz = to_fixed(uz, kVelocityTop);
   // c = c_j of the pair (i, j = i + 9): (c.u) (c.a) + P and c.b.  The products
   // round down, alike for i and j, so their momentum cancels; the rest population
-  // is what is left of the node's mass, which the collision then keeps exactly.
+  // is what is left of the node's mass.  The 19 integers keep that mass exactly,
+  // the doubles they become to their own rounding.
   int64_t left = M.mass;
   auto pair = [&](int i, int64_t cu, int64_t ca, int64_t cb, int64_t p) {
     const int64_t e = p + mul_high(cu, ca);
