@@ -837,7 +837,7 @@ MechPlan mech_plan(const hc_handle* h, const TypeSlot& ts) {
   if (cs == 8 && nv > 8 * 96 && 16 * n <= h->sms && ts.cluster16) cs = 16;
   const size_t whole = 4 * (6 * (size_t)nv + 7 * (size_t)nf + 3 * (size_t)ne * (model == HC_MODEL_PLT_SIMPLE ? 2 : 1)) +
                        (size_t)nv + 272;
-  if (h->tune[6] == 2 && nf < 65536 && ne < 65536 && (h->f64 || (whole <= 110 * 1024 && (h->tuned || !few_small(h))))) {
+  if (h->tune[6] == 2 && (h->f64 || (whole <= 110 * 1024 && (h->tuned || !few_small(h))))) {
     int c = cs;
     while (c < 8 && bytes(c) > (size_t)h->staged_limit) c *= 2;
     if (bytes(c) <= (size_t)h->staged_limit) {
@@ -1838,9 +1838,10 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
   };
   const size_t o_tris = put_i(c.tris), o_edges = put_i(c.edges), o_bt = put_i(c.bend_tris),
                o_bo = put_i(c.bend_outer), o_ring = put_i(c.ring), o_rn = put_i(c.ring_n), o_in = put_i(c.inner),
-               o_vf = put_i(c.vface), o_ve = put_i(c.vedge), o_vo = put_i(c.vopp), o_vio = put_i(c.vinner_off),
-               o_vi = put_i(c.vinner), o_sr = put_i(c.slot_rot);
-  // the packed tables (TypeDev), each from a 16-byte boundary
+               o_ve = put_i(c.vedge), o_vo = put_i(c.vopp), o_vio = put_i(c.vinner_off), o_vi = put_i(c.vinner);
+  // the packed tables (TypeDev), each from a 16-byte boundary.  Their 16-bit
+  // indices hold every type: with at most six edges a vertex, nf <= 2 nv and
+  // ne <= 3 nv, and the shared memory above limits nv to 9,300.
   auto align16 = [&] {
     while (iv.size() % 4) iv.push_back(0);
     return iv.size();
@@ -1858,10 +1859,8 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
     }
     return o;
   };
-  const bool narrow = c.nf < 65536 && c.ne < 65536;
-  const size_t o_r16 = put_six(c.ring, true), o_vf16 = narrow ? put_six(c.vface, false) : 0,
-               o_ve16 = narrow ? put_six(c.vedge, false) : 0, o_vo16 = narrow ? put_six(c.vopp, false) : 0,
-               o_t16 = align16();
+  const size_t o_r16 = put_six(c.ring, true), o_vf16 = put_six(c.vface, false), o_ve16 = put_six(c.vedge, false),
+               o_vo16 = put_six(c.vopp, false), o_t16 = align16();
   for (int k = 0; k < c.nf; ++k) {
     iv.push_back(c.tris[3 * k] | (int)((uint32_t)c.tris[3 * k + 1] << 16));
     iv.push_back(c.tris[3 * k + 2]);
@@ -1876,12 +1875,14 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
     return o;
   };
   const size_t o_a0 = put_d(c.tri_a0), o_l0 = put_d(c.edge_l0), o_ang = put_d(c.edge_angle0),
-               o_pd = put_d(c.patch_d0), o_il = put_d(c.inner_l0), o_sa = put_d(c.slot_a0), o_sl = put_d(c.slot_l0);
-  // the mixed form reads 32-bit copies, the plain form the reciprocals of the
-  // rest areas and lengths
+               o_pd = put_d(c.patch_d0), o_il = put_d(c.inner_l0);
+  // the mixed form reads 32-bit copies, and its slots' rest values from one
+  // table; the plain form also the reciprocals of the rest areas and lengths
   std::vector<float> fv;
-  size_t o_ia = 0, o_iel = 0, o_sf = 0;
+  size_t o_sa = 0, o_sl = 0, o_ia = 0, o_iel = 0, o_sf = 0;
   if (h->f64) {
+    o_sa = put_d(c.slot_a0);
+    o_sl = put_d(c.slot_l0);
     auto reciprocals = [](std::vector<double> a) {
       for (double& x : a) x = 1.0 / x;
       return a;
@@ -1922,19 +1923,16 @@ int hc_add_cell_type(hc_handle* h, const char* name, int model, const hc_materia
   d.ring = ibase + o_ring;
   d.ring_n = ibase + o_rn;
   d.inner = ibase + o_in;
-  d.vface = ibase + o_vf;
   d.vedge = ibase + o_ve;
   d.vopp = ibase + o_vo;
   d.vinner_off = ibase + o_vio;
   d.vinner = ibase + o_vi;
-  d.slot_rot = ibase + o_sr;
-  d.slot_a0 = dbase + o_sa;
-  d.slot_l0 = dbase + o_sl;
-  auto six = [&](size_t o) { return narrow ? (const uint4*)(ibase + o) : nullptr; };
+  d.slot_a0 = h->f64 ? dbase + o_sa : nullptr;
+  d.slot_l0 = h->f64 ? dbase + o_sl : nullptr;
   d.ring16 = (const uint4*)(ibase + o_r16);
-  d.vface16 = six(o_vf16);
-  d.vedge16 = six(o_ve16);
-  d.vopp16 = six(o_vo16);
+  d.vface16 = (const uint4*)(ibase + o_vf16);
+  d.vedge16 = (const uint4*)(ibase + o_ve16);
+  d.vopp16 = (const uint4*)(ibase + o_vo16);
   d.tris16 = (const uint2*)(ibase + o_t16);
   d.edges16 = (const uint32_t*)(ibase + o_e16);
   d.slot_f = h->f64 ? nullptr : (const float4*)(fbase + o_sf);
@@ -2450,9 +2448,9 @@ long long hc_estimate_device_bytes(const hc_params* p, int nvertices, int ncells
   b += vcap * (3 * 8 + 6 * ts + 3 * 4) + ccap * 4 * 4;
   // per-type rest-state blobs (hc_add_cell_type) and cell lists.  A closed mesh
   // has 2 faces and 3 edges a vertex, at most one inner link for two vertices:
-  // 81 ints, 21.5 doubles, and 5 doubles or 33.5 floats more; 16-byte alignment
+  // 69 ints, 9.5 doubles, and 17 doubles or 21.5 floats more; 16-byte alignment
   // of the tables within a blob
-  b += (f64 ? 536LL : 630LL) * nvertices + 128LL * hcd::MAX_TYPES + 4LL * ncells;
+  b += (f64 ? 488LL : 438LL) * nvertices + 128LL * hcd::MAX_TYPES + 4LL * ncells;
   // tile lists (hc_read_bins) and readback staging (hc_read_fluid, hc_read_vertices)
   const int tx = p->tile[0] > 0 ? p->tile[0] : 8, ty = p->tile[1] > 0 ? p->tile[1] : 8,
             tz = p->tile[2] > 0 ? p->tile[2] : 8;

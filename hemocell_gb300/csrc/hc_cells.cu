@@ -990,24 +990,6 @@ struct Face {
   V3t<T> cen;
 };
 
-template <typename T>
-__device__ __forceinline__ Face<T> face_geometry(const T* sx, const TypeDev& t, int k) {
-  const int i0 = t.tris[3 * k], i1 = t.tris[3 * k + 1], i2 = t.tris[3 * k + 2];
-  const V3t<T> v0 = ld3(sx, i0), v1 = ld3(sx, i1), v2 = ld3(sx, i2);
-  Face<T> F;
-  V3t<T> n = vcross(v1 - v0, v2 - v0);
-  const T nn = vnorm(n);
-  if (nn != T(0)) {
-    F.area = T(0.5) * nn;
-    F.n = {n.x / nn, n.y / nn, n.z / nn};
-  } else {
-    F.area = T(0);
-    F.n = {T(0), T(0), T(0)};
-  }
-  F.cen = {(v0.x + v1.x + v2.x) / T(3), (v0.y + v1.y + v2.y) / T(3), (v0.z + v1.z + v2.z) / T(3)};
-  return F;
-}
-
 // platelet dihedral bending force of edge e (pltSimpleModel.cpp:156-182),
 // +bfv on its end points, -bfv on the two outer points
 template <typename T>

@@ -127,18 +127,15 @@ struct TypeDev {
   const int* ring;        // nv*6
   const int* ring_n;      // nv
   const int* inner;       // ni*2
-  const int* vface;       // nv*6 per-vertex adjacency (see hc_host.h)
-  const int* vedge;       // nv*6
+  const int* vedge;       // nv*6 per-vertex adjacency (see hc_host.h)
   const int* vopp;        // nv*6
   const int* vinner_off;  // nv+1
   const int* vinner;
-  const int* slot_rot;    // nv*6
-  const double* slot_a0;  // nv*6
+  const double* slot_a0;  // nv*6 (FP64 handles only)
   const double* slot_l0;  // nv*6
   // The same tables in 16-bit indices, one 16-byte load a vertex (lane j of six;
   // the ring's lanes 6 and 7 hold ring_n and slot_rot in two bits each), one
-  // 8-byte load a face and one 4-byte load an edge.  vface16 and later need
-  // nf, ne < 65536 (null otherwise).
+  // 8-byte load a face and one 4-byte load an edge.
   const uint4* ring16;
   const uint4* vface16;
   const uint4* vedge16;
