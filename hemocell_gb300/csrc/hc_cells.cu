@@ -866,6 +866,18 @@ __device__ __forceinline__ V3t<T> unit_normal(V3t<T> a, V3t<T> b, V3t<T> c) {
   return {T(0), T(0), T(0)};
 }
 
+// Doubles at the start of the force assembly's shared memory: one partial sum a
+// warp of the largest block, the block's sum, the volume force and the same per area.
+template <typename T>
+constexpr int kMechThreads = sizeof(T) == 8 ? 384 : 768;
+template <typename T>
+constexpr int kSum = kMechThreads<T> / 32;
+template <typename T>
+constexpr int kVolumeForce = kSum<T> + 1;
+template <typename T>
+constexpr int kForcePerArea = kSum<T> + 2;
+template <typename T>
+constexpr int kMechHeader = kSum<T> + 3;
 template <typename T>
 __device__ __forceinline__ double block_sum(double v, double* red) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -876,10 +888,10 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
     const int nw = (blockDim.x + 31) >> 5;
     double s = lane < nw ? red[lane] : 0.0;
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) red[32] = s;
+    if (lane == 0) red[kSum<T>] = s;
   }
   __syncthreads();
-  return red[32];
+  return red[kSum<T>];
 }
 
 template <typename T>
@@ -899,12 +911,18 @@ __device__ __forceinline__ float rest_value<float>(const double*, const float* f
 __host__ __device__ __forceinline__ int cluster_chunk(int n, int cluster) {
   return ((n + cluster - 1) / cluster + 31) / 32 * 32;
 }
-constexpr int kClusterHeader = 40;
+// The vertex-centric kernel's shared memory: positions, the own bending forces and
+// the valences.  A cell on one CTA takes no more than its vertices: rounded up to
+// whole warps, the largest types (4,731 vertices in FP64, 9,273 in FP32) would not fit.
+__host__ __device__ __forceinline__ int gather_chunk(int nv, int cluster) {
+  return cluster == 1 ? nv : cluster_chunk(nv, cluster);
+}
 template <typename T>
 size_t mechanics_smem_bytes(int nv, int cluster) {
-  return kClusterHeader * sizeof(double) + (3 * (size_t)nv + 3 * (size_t)cluster_chunk(nv, cluster)) * sizeof(T) +
+  return kMechHeader<T> * sizeof(double) + (3 * (size_t)nv + 3 * (size_t)gather_chunk(nv, cluster)) * sizeof(T) +
          (size_t)nv;
 }
+constexpr int kStagedHeader = 40;  // of the staged kernel, whose faces start on a 16-byte boundary
 template <typename T>
 __device__ __forceinline__ V3t<T> ld3_cluster(uint32_t a) {
   V3t<T> v;
@@ -1156,7 +1174,7 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
   const long long V = vv.V;
   const int tid = threadIdx.x, bs = blockDim.x;
   constexpr bool kF64 = sizeof(T) == 8;
-  const int nv = t.nv, vch = cluster_chunk(nv, cs), fch = cluster_chunk(t.nf, cs);
+  const int nv = t.nv, vch = gather_chunk(nv, cs), fch = cluster_chunk(t.nf, cs);
   const int v0 = min(rank * vch, nv), v1 = min(v0 + vch, nv);
   const int f0 = min(rank * fch, t.nf), f1 = min(f0 + fch, t.nf);
   T* sbf = sx + 3 * nv;  // own bending force per own vertex
@@ -1228,20 +1246,20 @@ __device__ __forceinline__ void gather_cell(const MechView<T>& M, const TypeDev&
       q[2] = bf.z;
     }
   }
-  block_sum<T>(vol, red);  // red[32] = sum over the block
+  block_sum<T>(vol, red);  // red[kSum] = sum over the block
   cluster_sync(cs);
   const Chunked<false> bending(sbf, vch, 3 * sizeof(T));
   // volume constraint in FP64 (rbcHighOrderModel.cpp:100-104), by one thread
   if (tid == 0) {
-    const double volume = cluster_sum(red + 32, cs) * (1.0 / 6.0);
+    const double volume = cluster_sum(red + kSum<T>, cs) * (1.0 / 6.0);
     const double vfr = (volume - t.volume_eq) / t.volume_eq;
     const double vf = -t.k_volume * vfr / fabs(kMaxVol - vfr * vfr);
-    red[33] = vf;
-    red[31] = vf / t.area_mean_eq;
+    red[kVolumeForce<T>] = vf;
+    red[kForcePerArea<T>] = vf / t.area_mean_eq;
   }
   __syncthreads();
-  const T vforce = (T)red[33];
-  const T vforce_per_area = (T)red[31];
+  const T vforce = (T)red[kVolumeForce<T>];
+  const T vforce_per_area = (T)red[kForcePerArea<T>];
   const T area_mean = (T)t.area_mean_eq;
   const bool visc = (t.model != 0) || (t.eta_m != 0.0);
   // --- phase 2: gather per vertex
@@ -1386,7 +1404,7 @@ __device__ __forceinline__ void end_launch(const MechView<T>& M) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(sizeof(T) == 8 ? 384 : 768) k_mechanics(const MechView<T> M) {
+__global__ void __launch_bounds__(kMechThreads<T>) k_mechanics(const MechView<T> M) {
   extern __shared__ double smem_d[];
   __shared__ TypeDev tshared;
   __shared__ int hit;
@@ -1394,7 +1412,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 384 : 768) k_mechanics(const 
   for (int ci = blockIdx.x / cs; ci < M.ncells; ci += gridDim.x / cs) {
     const int cell = M.cells[ci], voff = M.cell_voff[cell];
     const bool alive = begin_cell(M, cell, voff, cs, rank, tshared, hit);
-    gather_cell(M, tshared, voff, alive, cs, rank, smem_d, reinterpret_cast<T*>(smem_d + kClusterHeader));
+    gather_cell(M, tshared, voff, alive, cs, rank, smem_d, reinterpret_cast<T*>(smem_d + kMechHeader<T>));
     cluster_sync(cs);  // no rank goes on or leaves while another reads its terms
   }
   end_launch(M);
@@ -1434,7 +1452,7 @@ template <typename T>
 __host__ __device__ __forceinline__ size_t staged_smem_bytes(int model, int nv, int nf, int ne, int cluster) {
   const size_t words = 5 * (size_t)cluster_chunk(nf, cluster) + 4 * (size_t)cluster_chunk(nv, cluster) + 3 * (size_t)nv +
                        (size_t)cluster_chunk(ne, cluster) * (model == 1 ? 4 : 1);
-  return kClusterHeader * sizeof(double) + words * sizeof(T);
+  return kStagedHeader * sizeof(double) + words * sizeof(T);
 }
 
 // x + x / |limit - x^2|, the saturating response of every membrane term
@@ -1476,7 +1494,7 @@ __global__ void __launch_bounds__(384, 2) k_mechanics_staged(const MechView<T> M
   const int f0 = min(rank * fch, nf), f1 = min(f0 + fch, nf);
   const int e0 = min(rank * ech, ne), e1 = min(e0 + ech, ne);
   double* red = smem_cluster;
-  T* sface = reinterpret_cast<T*>(smem_cluster + kClusterHeader);
+  T* sface = reinterpret_cast<T*>(smem_cluster + kStagedHeader);
   T* sinv = sface + 4 * fch;
   T* sbf = sinv + fch;
   T* sedge = sbf + 4 * vch;
@@ -1544,7 +1562,7 @@ __global__ void __launch_bounds__(384, 2) k_mechanics_staged(const MechView<T> M
       p[2] = pb.z;
     }
   }
-  block_sum<T>(vol, red);  // red[32] = the own faces' sum
+  block_sum<T>(vol, red);  // red[kSum] = the own faces' sum
   cluster_sync(cs);
   using Terms = Chunked<ONE>;
   const Terms faces(sface, fch, 4 * sizeof(T)), edges(sedge, ech, sizeof(T)), dihedral(splt, ech, 3 * sizeof(T)),
@@ -1555,9 +1573,9 @@ __global__ void __launch_bounds__(384, 2) k_mechanics_staged(const MechView<T> M
   // for it, so there are no divisions in it (960 FP32 cells 127 us with, 122
   // without)
   if (tid == 0) {
-    const double sum = ONE ? red[32] : cluster_sum(red + 32, cs);
+    const double sum = ONE ? red[kSum<T>] : cluster_sum(red + kSum<T>, cs);
     const double vfr = (sum * (1.0 / 6.0) - t.volume_eq) * t.inv_volume_eq;
-    red[33] = -t.k_volume * vfr * hcnewton::recip(fabs(kMaxVol - vfr * vfr)) * t.inv_area_mean_eq;
+    red[kVolumeForce<T>] = -t.k_volume * vfr * hcnewton::recip(fabs(kMaxVol - vfr * vfr)) * t.inv_area_mean_eq;
   }
   // --- own bending forces, from the unit normals of the incident faces
   if (!plt) {
@@ -1596,7 +1614,7 @@ __global__ void __launch_bounds__(384, 2) k_mechanics_staged(const MechView<T> M
     }
   }
   cluster_sync(cs);
-  const T push = T(0.5) * (T)red[33];  // volume force per cross product
+  const T push = T(0.5) * (T)red[kVolumeForce<T>];  // volume force per cross product
   // --- gather the own vertices' forces
   for (int iw = v0 + (tid & ~31); iw < v1; iw += bs) {
     // whole warps, whose last one's spare lanes repeat its last vertex
@@ -1686,12 +1704,12 @@ size_t mechanics_staged_bytes(int model, int nv, int nf, int ne, int cluster, bo
 // every inner link as one merged item loop.  Forces accumulate in shared
 // memory and are written once.
 template <typename T>
-__global__ void __launch_bounds__(sizeof(T) == 8 ? 384 : 768) k_mechanics_scatter(const MechView<T> M) {
+__global__ void __launch_bounds__(kMechThreads<T>) k_mechanics_scatter(const MechView<T> M) {
   pdl_wait();
   extern __shared__ double smem_d[];
   __shared__ TypeDev tshared;
-  double* red = smem_d;  // 34 doubles
-  T* sx = reinterpret_cast<T*>(smem_d + 34);
+  double* red = smem_d;
+  T* sx = reinterpret_cast<T*>(smem_d + kMechHeader<T>);
   const VertexView<T>& vv = M.vv;
   const long long V = vv.V;
   const int tid = threadIdx.x, bs = blockDim.x;
@@ -1935,7 +1953,7 @@ template <typename T>
 cudaError_t launch_mechanics(const MechView<T>& M, int cluster, int bs, int grid, int variant, cudaStream_t s) {
   if (M.ncells <= 0) return cudaSuccess;
   if (bs <= 0) bs = 256;
-  if (bs > (sizeof(T) == 8 ? 384 : 768)) bs = sizeof(T) == 8 ? 384 : 768;
+  if (bs > kMechThreads<T>) bs = kMechThreads<T>;
   if (grid <= 0 || grid > M.ncells) grid = M.ncells;
   if (variant == 1) return launch_kernel(k_mechanics_scatter<T>, dim3(grid), dim3(bs), M.dyn_smem, s, M.L.pdl, M);
   return launch_cluster(k_mechanics<T>, cluster, dim3(grid * cluster), dim3(bs), M.dyn_smem, s, M.L.pdl, M.carveout, M);
