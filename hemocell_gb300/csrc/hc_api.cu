@@ -99,7 +99,7 @@ struct hc_handle {
   int iter = 0;
   int velocity_every = 1;
   // k1 bx (0: row-staged, blocks of whole x-rows), k1 by, spread bs, ibm bs, mech bs, mech grid,
-  // mech variant (0 vertex gather, 1 face/edge scatter)
+  // mech variant (0 vertex gather, 1 face/edge scatter, 2 staged gather)
   int tune[8] = {64, 2, 128, 128, 384, 0, 0, 0};
   bool tuned = false;  // tune is the caller's (hc_set_tuning, hc_autotune), not the rules' (apply_rules)
   int sms = 1;         // SMs of the device
@@ -383,7 +383,14 @@ VertexView<T> vertex_view(hc_handle* h) {
 //   (50^3 box 56; every node 62, packed 58; pipe 289, 295, 287).
 //   Programmatic launch always (FP64 50^3 box 56 against 67, FP32 32^3 box 25.6
 //   against 25.7).
-//   Force assembly: variant 2 (see mech_plan).
+//   Force assembly: variant 2, or 0 for a handful of small FP32 cells (see
+//   mech_plan).
+bool few_small(const hc_handle* h) {
+  if (h->ncells > 16) return false;
+  for (const TypeSlot& ts : h->types)
+    if (!ts.cells.empty() && ts.tc.nv > 256) return false;
+  return true;
+}
 void apply_rules(hc_handle* h) {
   if (h->tuned) return;
   const int rule[8] = {64, 4, 128, 128, 384, 0, 2, 0x400};
@@ -399,6 +406,7 @@ void apply_rules(hc_handle* h) {
     if (h->nfluid > 0) h->tune[7] |= 0x100;
     return;
   }
+  if (few_small(h)) h->tune[6] = 0;
   if (!fast32) return;
   if (h->nfluid > 0 && 152LL * h->nfluid <= 64 << 20) h->tune[7] |= 0x2000;
   if (24LL * h->nvert >= h->N) h->tune[7] |= 0x300;
@@ -811,12 +819,6 @@ size_t gather_bytes(const hc_handle* h, const TypeSlot& ts, int cluster = 1) {
 // terms do not fit at all and, unless the caller chose the variant, a handful of
 // small cells: they take the same time either way, and the vertex-centric
 // kernel's spread adds in the same order from run to run.
-bool few_small(const hc_handle* h) {
-  if (h->ncells > 16) return false;
-  for (const TypeSlot& ts : h->types)
-    if (!ts.cells.empty() && ts.tc.nv > 256) return false;
-  return true;
-}
 struct MechPlan {
   bool staged;
   int cluster, bs;
@@ -837,7 +839,7 @@ MechPlan mech_plan(const hc_handle* h, const TypeSlot& ts) {
   if (cs == 8 && nv > 8 * 96 && 16 * n <= h->sms && ts.cluster16) cs = 16;
   const size_t whole = 4 * (6 * (size_t)nv + 7 * (size_t)nf + 3 * (size_t)ne * (model == HC_MODEL_PLT_SIMPLE ? 2 : 1)) +
                        (size_t)nv + 272;
-  if (h->tune[6] == 2 && (h->f64 || (whole <= 110 * 1024 && (h->tuned || !few_small(h))))) {
+  if (h->tune[6] == 2 && (h->f64 || whole <= 110 * 1024)) {
     int c = cs;
     while (c < 8 && bytes(c) > (size_t)h->staged_limit) c *= 2;
     if (bytes(c) <= (size_t)h->staged_limit) {
@@ -872,7 +874,7 @@ int enq_types(hc_handle* h, hcd::MechView<T> M, bool forced, bool all_due) {
     long long n, vertices;
   };
   std::vector<Launch> launches;
-  const bool together = h->tune[6] == 2 && all_due;
+  const bool together = (h->tune[6] == 2 || !h->tuned) && all_due;
   for (const TypeSlot& ts : h->types)
     if (!ts.cells.empty() && (forced || h->iter % ts.every == 0))
       launches.push_back({mech_plan(h, ts), ts.dcells, (long long)ts.cells.size(), (long long)ts.cells.size() * ts.tc.nv});
@@ -2536,6 +2538,7 @@ int hc_set_tuning(hc_handle* h, const int* in8) {
   }
   int old_tune[8];
   std::memcpy(old_tune, h->tune, sizeof(old_tune));
+  if (std::memcmp(old_tune, in8, sizeof(old_tune)) == 0) return HC_OK;  // the rules', or the caller's already
   std::memcpy(h->tune, in8, sizeof(h->tune));
   h->tuned = true;
   invalidate_graph(h);

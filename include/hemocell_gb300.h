@@ -277,7 +277,8 @@ int hc_device_status(hc_handle* h, unsigned int* status);
 int hc_autotune(hc_handle* h, const char* cache_path);
 int hc_get_tuning(hc_handle* h, int* out8);
 /* until hc_set_tuning or hc_autotune, the launch shapes follow the lattice and
- * its cells; hc_get_tuning returns the ones in use.
+ * its cells, whenever those change; hc_get_tuning returns the ones in use, and
+ * hc_set_tuning with those changes nothing.  Any other choice is kept as it is.
  * in8: collide-stream block (bx, by; bx = 0 whole rows, else 8 or 16, whose
  * warps are 8 x 4 or 16 x 2 tiles, or a multiple of 32; whole warps, at most
  * 256 threads), spread block,
