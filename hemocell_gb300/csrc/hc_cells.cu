@@ -1476,6 +1476,9 @@ __device__ __forceinline__ T inv_valence(int n) {
 // a / b by a reciprocal: fast in both forms
 __device__ __forceinline__ float quotient(float a, float b) { return fdiv(a, b); }
 __device__ __forceinline__ double quotient(double a, double b) { return a * hcnewton::recip(b); }
+// the same, rounded in FP32
+__device__ __forceinline__ float ratio(float a, float b) { return a / b; }
+__device__ __forceinline__ double ratio(double a, double b) { return quotient(a, b); }
 template <typename T, bool ONE>
 __global__ void __launch_bounds__(384, 2) k_mechanics_staged(const MechView<T> M) {
   extern __shared__ __align__(16) double smem_cluster[];
@@ -1656,23 +1659,24 @@ __global__ void __launch_bounds__(384, 2) k_mechanics_staged(const MechView<T> M
       const int e = t.vinner[q];
       const int o = t.inner[2 * e] == i ? t.inner[2 * e + 1] : t.inner[2 * e];
       const V3t<T> ev = ld3(sx, o) - xi;
+      // the forces follow the small difference of two lengths: the rounded root and
+      // quotients in FP32, as in the vertex-centric kernel (the same bits)
       T inv, len;
+      V3t<T> uv;  // toward the partner
       if constexpr (sizeof(T) == 8) {
         hcnewton::inv_length(vdot(ev, ev), inv, len);
+        uv = vscale(ev, inv);
       } else {
-        // the strain is the difference of nearly equal lengths: the rounded root,
-        // as in the vertex-centric kernel
         len = vnorm(ev);
-        inv = T(1) / len;
+        uv = {ev.x / len, ev.y / len, ev.z / len};
       }
-      const V3t<T> uv = vscale(ev, inv);  // toward the partner
       if (plt) {
         const T l0 = rest_value<T>(t.inner_l0, t.inner_l0f, e);
-        f = f + vscale(uv, (T)t.k_link * T(5) * quotient(len - l0, l0));
+        f = f + vscale(uv, (T)t.k_link * T(5) * ratio(len - l0, l0));
       } else if (t.model == 2) {
         const T d1 = T(2) * (T)t.radius, d2 = T(2) * (T)t.core_radius;
-        if (len < d1) f = f - vscale(uv, (T(1) - quotient(len, d1)) * (T)t.k_cyto);
-        if (len < d2) f = f - vscale(uv, (T(1) - quotient(len, d2)) * (T)t.k_inner_rigid);
+        if (len < d1) f = f - vscale(vscale(uv, T(1) - ratio(len, d1)), (T)t.k_cyto);
+        if (len < d2) f = f - vscale(vscale(uv, T(1) - ratio(len, d2)), (T)t.k_inner_rigid);
       }
     }
     if (on) {
