@@ -103,6 +103,7 @@ struct hc_handle {
   int tune[8] = {64, 2, 128, 128, 384, 0, 0, 0};
   bool tuned = false;  // tune is the caller's (hc_set_tuning, hc_autotune), not the rules' (apply_rules)
   int sms = 1;         // SMs of the device
+  int l2 = 0;          // bytes of its L2
   int staged_limit = 0;  // dynamic shared memory the staged force assembly may take
   // repulsion (setRepulsion / enableBoundaryParticles): constants, cutoffs in
   // lattice units, timescales (0 = off) and device state
@@ -373,9 +374,11 @@ VertexView<T> vertex_view(hc_handle* h) {
 //   In FP32: (x, y)-blocks, or the list where rows rounded up to warps idle a
 //   twentieth of their lanes (pipe, rows of 64: 84 against 89; of 97: 29 against
 //   32; of 181: 65 against 67).  Evict-last population stores while both buffers
-//   take at most half the L2 (61x59x131 pipe with repulsion 22.4 against 22.9 ms
-//   for 400 steps); beyond it they cost (pipe 83.5 against 82.2, the 181x117x93
-//   channel 65.7 against 63.6, the 128^3 suspension the same 212).
+//   take at most half the device's L2 (61x59x131 pipe with repulsion 22.5 against
+//   22.7 ms for 400 steps); beyond it they cost (pipe 83.5 against 82.2, the
+//   181x117x93 channel 65.7 against 63.6, the 128^3 suspension the same 212).  The
+//   handle decides for itself alone: eight small ones side by side, which together
+//   mark more than the L2 holds, take 22.7 against 22.5 ms.
 //   Node velocity in FP32: every fluid node from one vertex for 24 nodes on (96^3
 //   with 80 RBCs 71 against 72; with 20 60 against 68 the other way), else the
 //   tagged nodes packed into warps from half a million nodes on (128^3 with 6
@@ -408,7 +411,7 @@ void apply_rules(hc_handle* h) {
   }
   if (few_small(h)) h->tune[6] = 0;
   if (!fast32) return;
-  if (h->nfluid > 0 && 152LL * h->nfluid <= 64 << 20) h->tune[7] |= 0x2000;
+  if (h->nfluid > 0 && 2 * 152LL * h->nfluid <= h->l2) h->tune[7] |= 0x2000;
   if (24LL * h->nvert >= h->N) h->tune[7] |= 0x300;
   else if (h->N >= 500000) h->tune[7] |= 0x200;
 }
@@ -814,11 +817,17 @@ size_t gather_bytes(const hc_handle* h, const TypeSlot& ts, int cluster = 1) {
 //         n = 110: 28 / 35 / 41 / 65    280: 39 / 68 / 108 / 130
 // Threads, staged: one per face of the CTA's share, 128 to 384 (256 from four
 // CTAs a cell on); the 384 of a whole RBC are two CTAs an SM.
-// An FP32 type whose terms, face by face and edge by edge, took more than 110 KB
-// in one CTA (a 2562-vertex WBC) is assembled vertex by vertex, as is one whose
-// terms do not fit at all and, unless the caller chose the variant, a handful of
-// small cells: they take the same time either way, and the vertex-centric
-// kernel's spread adds in the same order from run to run.
+// An FP32 type whose terms, kept face by face and edge by edge as vectors, would
+// take more than 110 KB in one CTA (above 960 vertices of a red or white cell, 730
+// of a platelet) is assembled vertex by vertex.  That is the line of an earlier
+// layout; at the one size in use beyond it, the 2562-vertex white cell, both
+// kernels take the same time (128^3 suspension with two of them, 300 steps: 69.7 ms
+// each).  So is a type whose terms do not fit at all, and, by the rules, a handful
+// of small cells: red cells alone 22 us a step against 24 staged; with platelets,
+// whose dihedral terms it computes once for each incident vertex, 34 against 26.
+// Nothing orders either kernel's spread (two runs' velocities are 4e-8 apart), but
+// for such a handful the vertex-centric one repeats positions to 1e-9 over 21
+// steps, where the staged one's were 9e-9 apart.
 struct MechPlan {
   bool staged;
   int cluster, bs;
@@ -833,8 +842,10 @@ MechPlan mech_plan(const hc_handle* h, const TypeSlot& ts) {
   if (h->f64) cs = 8 * n <= 2 * h->sms ? 8 : (4 * n <= (used_types(h) > 1 ? 2 : 3) * h->sms ? 4 : 2);
   else
     while (cs < 8 && 2 * n * cs <= h->sms) cs *= 2;
-  // with the spread in it, CTAs of one cell add to the same nodes in whatever
-  // order they arrive: a cell that one round of a CTA's threads holds stays whole
+  // with the advance and the spread in it, a cell that one round of a CTA's threads
+  // holds stays whole (against clusters, us a step: FP64, 8 cells of 42 vertices 34
+  // and 40, 16 of 162 the same 41, with platelets 42 and 43; FP32, 40 of 162
+  // vertices 24.6 and 29.7)
   if (h->p.launch == HC_LAUNCH_BATCHED && nv <= 256) cs = 1;
   if (cs == 8 && nv > 8 * 96 && 16 * n <= h->sms && ts.cluster16) cs = 16;
   const size_t whole = 4 * (6 * (size_t)nv + 7 * (size_t)nf + 3 * (size_t)ne * (model == HC_MODEL_PLT_SIMPLE ? 2 : 1)) +
@@ -1668,6 +1679,7 @@ hc_handle* hc_create(const hc_params* p) {
   cudaMemsetAsync(h->status, 0, sizeof(unsigned int), h->stream);
   h->hflag.assign(h->N, 0);
   cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, p->device);
+  cudaDeviceGetAttribute(&h->l2, cudaDevAttrL2CacheSize, p->device);
   if (upload_flags(h) != HC_OK) return bail(h->err);
   if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return bail(cudaGetErrorString(e));
   return h;
