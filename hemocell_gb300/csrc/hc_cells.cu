@@ -185,7 +185,10 @@ __device__ __forceinline__ void ibm_weights(const LbmView<T>& L, double px, doub
   }
   // The weights of a whole stencil sum to one by themselves, to the rounding
   // of their products: FP64, whose pipe bounds the cell kernels, renormalises
-  // only a stencil that lost a node (24 of its 60 instructions otherwise).
+  // only a stencil that lost a node (24 of its 60 instructions otherwise).  Random
+  // coordinates up to 1000, rms in units of 2^-53 against exact weights: each
+  // weight 0.115 off (renormalised 0.181), their sum 0.35 (0.82), the value
+  // interpolated from a random field 0.64 (0.75).
   if (kF64 && cut) {
 #pragma unroll
     for (int s = 0; s < 8; ++s) total += K.w[s];
@@ -197,8 +200,9 @@ __device__ __forceinline__ void ibm_weights(const LbmView<T>& L, double px, doub
   }
 }
 
-// Bit s of corner[n]: slot s of the 2x2x2 block from node n on is a boundary
-// node (unset beyond a non-periodic end, which the callers see themselves).
+// Bit s of corner[n]: slot s of the 2x2x2 block from node n on, wrapped at the
+// lattice's ends, is a boundary node.  Of a slot beyond a non-periodic end the bit
+// says nothing; the callers leave such a slot out by its index.
 __global__ void k_corner_flags(const uint8_t* flag, uint8_t* corner, int nx, int ny, int nz) {
   const int X = blockIdx.x * blockDim.x + threadIdx.x;
   if (X >= nx) return;
