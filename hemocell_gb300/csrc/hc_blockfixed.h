@@ -11,7 +11,7 @@
 // moments round to 2^-53 of the largest and enter every population, is no closer:
 // whole runs are a tenth as far off (tests/lattice_error_check.cpp).  Sums, the pair
 // terms and the relaxation run on those integers; the scalars of a node (1/rho, u,
-// the even part, the force's shares) stay in FP64: 30 FP64 instructions a node
+// the even part, the force's shares) stay in FP64: 27 FP64 instructions a node
 // instead of 143.
 //
 // Bounds: |v| < 2^(top + 1) for every population and force component, so the
