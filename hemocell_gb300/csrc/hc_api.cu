@@ -369,8 +369,8 @@ VertexView<T> vertex_view(hc_handle* h) {
 // hc_autotune), from its lattice and cells.  Steps in microseconds, this choice
 // against the other side of the line:
 //   Collide-stream in FP64: over the fluid-node list, as a warp with one fluid
-//   node costs the issue slots as much as a full one (pipe 64x64x256 82 against
-//   110 for the kernel, 150^3 Couette box 338 against 384).
+//   node costs the issue slots as much as a full one (pipe 64x64x256 84 against
+//   111 for the kernel, 150^3 Couette box 342 against 391).
 //   In FP32: (x, y)-blocks, or the list where rows rounded up to warps idle a
 //   twentieth of their lanes (pipe, rows of 64: 84 against 89; of 97: 29 against
 //   32; of 181: 65 against 67).  Evict-last population stores while both buffers

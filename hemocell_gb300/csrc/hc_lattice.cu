@@ -109,7 +109,8 @@ __device__ __noinline__ void collide_refused(const LbmView<double>& L, Idx n, in
 // FP64 runs in block fixed point (hc_blockfixed.h): the FP64 pipe bounded the
 // kernel at 143 instructions a node (206 before the pair terms shared c.u).  The
 // pipe 64x64x256: 371 us by equilibrium and source, 206 in FP64 over the fluid
-// list, 83 now; the 150^3 Couette box 1620, 904 and 338 us.
+// list, 84 now; the 150^3 Couette box 1620, 904 and 342 us (338
+// with omega/12 in 53 bits, whose runs drifted: hc_blockfixed.h).
 template <typename T, typename Idx, bool KEEP = false>
 __device__ __forceinline__ void collide_store(const LbmView<T>& L, Idx n, int X, int Y, int Z, uint32_t m,
                                               const T f[19], T Fx, T Fy, T Fz) {

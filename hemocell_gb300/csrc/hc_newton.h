@@ -12,8 +12,8 @@
 // (Householder, The Numerical Treatment of a Single Nonlinear Equation, 1970).
 // For a seed within 2^-19 the relative error stays below 2^-52: 2^-53 of the last
 // rounding, at most 2^-54 of t's, and e0^3 or 5/16 (2 e0)^3 of the iteration.  A
-// CPU test checks that over random arguments and seeds.  Host and device compile
-// the same steps.
+// CPU test checks that over random arguments and seeds, a GPU test with the
+// hardware's seeds over all binades.  Host and device compile the same steps.
 #pragma once
 #include <math.h>
 #include <stdint.h>
